@@ -15,7 +15,7 @@
 // 1/(x-Ia) = (x+Ia)(x^2-a^2)/D_j, 1/(x+Ia) = (x-Ia)(x^2-a^2)/D_j.  The batch inversion then
 // runs over n/4 values and the whole vector costs about 6 multiplications per weight
 // instead of 13.
-#include "common.cuh"
+#include "block.cuh"
 
 namespace gzk
 {
@@ -120,7 +120,11 @@ namespace gzk
                 if (has_s) suf[t] = mul(s, so);
                 __syncthreads();
             }
-            if (t == 0) total_inv = inv(pre[kInvThreads - 1]);
+            if (t < 32)
+            {
+                const Fr inverse = inv_quad<FrCfg>(pre[kInvThreads - 1]);
+                if (t == 0) total_inv = inverse;
+            }
             __syncthreads();
             // 1 / (own run product) = total_inv * prod_{t' < t} * prod_{t' > t}
             Fr outer = total_inv;
@@ -342,26 +346,11 @@ namespace gzk
         // node-domain weights every binding of the flow asks for) is one dependent chain, so it takes one
         // quartet per thread and spreads over as many SMs as it has 256-quartet groups; a large domain
         // takes four and amortises the serial inversion over 1024 quartets.
-        struct FusedShared
-        {
-            Fr warp_incl[kThreads / 32];
-            Fr warp_pre[kThreads / 32];
-            Fr warp_suf[kThreads / 32];
-            Fr cta_inverse;
-        };
-
         template <int ELEMS>
-        __device__ __forceinline__ void bary4_fused_body(const BaryArgs& a, Fr* out, int* status, FusedShared& sh)
+        __device__ __forceinline__ void bary4_fused_body(const BaryArgs& a, Fr* out, int* status, BatchInvertShared<kThreads>& sh)
         {
-            Fr* warp_incl = sh.warp_incl;
-            Fr* warp_pre = sh.warp_pre;
-            Fr* warp_suf = sh.warp_suf;
-            Fr& cta_inverse = sh.cta_inverse;
             const uint32_t chunk = blockIdx.x < a.kept_blocks ? blockIdx.x : a.last_chunk;
             const uint64_t base = static_cast<uint64_t>(chunk) * (kThreads * ELEMS);
-            const int lane = threadIdx.x & 31;
-            const int warp = threadIdx.x >> 5;
-
             Fr d[ELEMS], pre[ELEMS];
             Fr mine = Fr::one();
 #pragma unroll
@@ -373,43 +362,9 @@ namespace gzk
                 pre[j] = mine;
                 mine = mul(mine, d[j]);
             }
-            Fr incl = mine, sufx = mine;
-#pragma unroll
-            for (int offset = 1; offset < 32; offset <<= 1)
-            {
-                const Fr up = shfl_fr(incl, (lane - offset) & 31);
-                const Fr down = shfl_fr(sufx, (lane + offset) & 31);
-                if (lane >= offset) incl = mul(incl, up);
-                if (lane + offset < 32) sufx = mul(sufx, down);
-            }
-            Fr left = shfl_fr(incl, (lane - 1) & 31);
-            Fr right = shfl_fr(sufx, (lane + 1) & 31);
-            if (lane == 0) left = Fr::one();
-            if (lane == 31) right = Fr::one();
-            if (lane == 31) warp_incl[warp] = incl;
-            __syncthreads();
-            if (threadIdx.x == 0)
-            {
-                Fr run = Fr::one();
-#pragma unroll
-                for (int w = 0; w < kThreads / 32; ++w)
-                {
-                    warp_pre[w] = run;
-                    run = mul(run, warp_incl[w]);
-                }
-                const Fr total = run;
-                run = Fr::one();
-#pragma unroll
-                for (int w = kThreads / 32 - 1; w >= 0; --w)
-                {
-                    warp_suf[w] = run;
-                    run = mul(run, warp_incl[w]);
-                }
-                if (total.is_zero()) raise_status(status, GZK_E_DOMAIN, 103);
-                cta_inverse = inv(total);
-            }
-            __syncthreads();
-            const Fr outer = mul(cta_inverse, mul(mul(left, warp_pre[warp]), mul(right, warp_suf[warp])));
+            bool zero = false;
+            const Fr outer = block_batch_invert<kThreads>(mine, sh, &zero);
+            if (zero && threadIdx.x == 0) raise_status(status, GZK_E_DOMAIN, 103);
             Fr rest = mul(a.scale, outer);  // (x^n-1)/n over the product of the thread's denominators 0 .. j
 #pragma unroll
             for (int j = ELEMS - 1; j >= 0; --j)
@@ -443,7 +398,7 @@ namespace gzk
         template <int ELEMS>
         __global__ void __launch_bounds__(kThreads, 2) bary4_fused_kernel(BaryArgs a, Fr* out, int* status)
         {
-            __shared__ FusedShared sh;
+            __shared__ BatchInvertShared<kThreads> sh;
             bary4_fused_body<ELEMS>(a, out, status, sh);
         }
 
@@ -457,7 +412,7 @@ namespace gzk
         };
         __global__ void __launch_bounds__(kThreads, 2) bary4_fused_multi_kernel(BaryMultiArgs m, int* status)
         {
-            __shared__ FusedShared sh;
+            __shared__ BatchInvertShared<kThreads> sh;
             bary4_fused_body<1>(m.point[blockIdx.y], m.out[blockIdx.y], status, sh);
         }
     }

@@ -4,6 +4,7 @@
 #pragma once
 
 #include "common.cuh"
+#include "inverse.cuh"
 
 namespace gzk
 {
@@ -86,6 +87,62 @@ namespace gzk
         }
         __syncthreads();
         return total;
+    }
+
+    // Shared memory of a CTA-wide batch inversion.
+    template <int THREADS>
+    struct BatchInvertShared
+    {
+        Fr warp_products[THREADS / 32];
+        Fr inverse;
+    };
+
+    // Returns 1/mine for every thread of the CTA through ONE inversion of the product over the CTA; *zero
+    // (thread 0 only) tells that this product was zero.  Products run over an xor butterfly: after the step
+    // with offset o a lane holds the product of its block of 2o lanes and, in `others`, that product without
+    // its own value, so a step costs two multiplications and nothing is undone afterwards; the warp products
+    // go through the same butterfly in every warp, which leaves warp 0 with the total it inverts (a chain of
+    // 10 + 5 multiplications around the inversion at 256 threads; a prefix and a suffix scan with the warp
+    // products in sequence take 10 + 16 + 5).
+    template <int THREADS>
+    __device__ __forceinline__ Fr block_batch_invert(const Fr& mine, BatchInvertShared<THREADS>& sh, bool* zero)
+    {
+        constexpr int W = THREADS / 32;
+        static_assert((W & (W - 1)) == 0 && W <= 32, "whole power-of-two number of warps");
+        const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+        Fr others = shfl_fr_idx(mine, lane ^ 1);
+        Fr product = mul(mine, others);
+#pragma unroll 1
+        for (int offset = 2; offset < 32; offset <<= 1)
+        {
+            const Fr sibling = shfl_fr_idx(product, lane ^ offset);
+            others = mul(others, sibling);
+            product = mul(product, sibling);
+        }
+        if (W > 1)
+        {
+            if (lane == 0) sh.warp_products[warp] = product;
+            __syncthreads();
+            // lane l works on warp product l mod W
+            product = sh.warp_products[lane & (W - 1)];
+            Fr warp_others = Fr::one();
+#pragma unroll 1
+            for (int offset = 1; offset < W; offset <<= 1)
+            {
+                const Fr sibling = shfl_fr_idx(product, lane ^ offset);
+                warp_others = offset == 1 ? sibling : mul(warp_others, sibling);
+                product = mul(product, sibling);
+            }
+            others = mul(others, shfl_fr_idx(warp_others, warp));
+        }
+        *zero = product.is_zero();
+        if (warp == 0)
+        {
+            const Fr inverse = inv_quad<FrCfg>(product);
+            if (lane == 0) sh.inverse = inverse;
+        }
+        __syncthreads();
+        return mul(sh.inverse, others);
     }
 
     // Given each thread's product `mine` and the inverse of the product over

@@ -103,8 +103,7 @@ namespace gzk
         // main pass on its own (each CTA inverts the product of its 512 denominators).
         __global__ void __launch_bounds__(kThreads) shifted_inverse_kernel(ScanArgs a, Fr* inv_out)
         {
-            __shared__ Fr slots[3 * kWarps];
-            __shared__ Fr local_inverse;
+            __shared__ BatchInvertShared<kThreads> sh;
             const uint64_t base = static_cast<uint64_t>(blockIdx.x) * kChunk + static_cast<uint64_t>(threadIdx.x) * kElems;
             Fr d[kElems], pre[kElems];
             Fr mine = Fr::one();
@@ -116,14 +115,9 @@ namespace gzk
                 pre[j] = mine;
                 mine = mul(mine, d[j]);
             }
-            const Fr total = block_product<kThreads>(mine, slots);
-            if (threadIdx.x == 0)
-            {
-                if (total.is_zero()) raise_status(a.status, GZK_E_DOMAIN, 1404);
-                local_inverse = inv(total);
-            }
-            __syncthreads();
-            Fr rest = block_invert_products<kThreads>(mine, local_inverse, slots);
+            bool zero = false;
+            Fr rest = block_batch_invert<kThreads>(mine, sh, &zero);
+            if (zero && threadIdx.x == 0) raise_status(a.status, GZK_E_DOMAIN, 1404);
 #pragma unroll
             for (int j = kElems - 1; j >= 0; --j)
             {
@@ -184,7 +178,7 @@ namespace gzk
         struct MainShared
         {
             Fr slots[3 * kWarps];
-            Fr local_inverse;
+            BatchInvertShared<kThreads> invert;
             SegVal seg_slots[kWarps];
             uint32_t first_flag;
         };
@@ -193,8 +187,6 @@ namespace gzk
         template <int OP, bool LOCAL_INV>
         __device__ __forceinline__ void scan_main_body(const ScanArgs& a, uint32_t block, MainShared& sh)
         {
-            Fr* slots = sh.slots;
-            Fr& local_inverse = sh.local_inverse;
             SegVal* seg_slots = sh.seg_slots;
             uint32_t& first_flag = sh.first_flag;
             const uint64_t base = static_cast<uint64_t>(block) * kChunk + static_cast<uint64_t>(threadIdx.x) * kElems;
@@ -220,24 +212,17 @@ namespace gzk
                     pre[j] = mine;
                     mine = mul(mine, d[j]);
                 }
-                Fr cta_inverse;
+                Fr rest;  // inverse of the product of the thread's rows 0 .. j
                 if (LOCAL_INV)
                 {
-                    const Fr total = block_product<kThreads>(mine, slots);
-                    if (threadIdx.x == 0)
-                    {
-                        if (total.is_zero()) raise_status(a.status, GZK_E_DOMAIN, 1402);
-                        local_inverse = inv(total);
-                    }
-                    __syncthreads();
-                    cta_inverse = local_inverse;
+                    bool zero = false;
+                    rest = block_batch_invert<kThreads>(mine, sh.invert, &zero);
+                    if (zero && threadIdx.x == 0) raise_status(a.status, GZK_E_DOMAIN, 1402);
                 }
                 else
                 {
-                    cta_inverse = load_fr(a.cta_products + block);
+                    rest = block_invert_products<kThreads>(mine, load_fr(a.cta_products + block), sh.slots);
                 }
-                const Fr outer = block_invert_products<kThreads>(mine, cta_inverse, slots);
-                Fr rest = outer;  // inverse of the product of the thread's rows 0 .. j
 #pragma unroll
                 for (int j = kElems - 1; j >= 0; --j)
                 {
