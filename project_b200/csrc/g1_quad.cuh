@@ -34,7 +34,7 @@ namespace gzk
     }
     // One multiplication for all callers: inlined twenty times over, a kernel that runs once per call would spend
     // its time fetching instructions.
-    __device__ __noinline__ Fp quad_mul(const Fp a, const Fp b) { return mul(a, b); }
+    static __device__ __noinline__ Fp quad_mul(const Fp a, const Fp b) { return mul(a, b); }
 
     // The component of this lane of an affine point, or of the point at infinity (0, 0) where it is that or `take`
     // is false; called by whole warps.
@@ -48,7 +48,7 @@ namespace gzk
     }
 
     // p + q and its doubling as one lane computes them (operands that coincide; the sum that vanishes)
-    __device__ __noinline__ Fp quad_add_special(const Fp p, const Fp q)
+    static __device__ __noinline__ Fp quad_add_special(const Fp p, const Fp q)
     {
         const int lane = threadIdx.x & 31, quad = lane & ~3, role = lane & 3;
         G1Xyzz a, b;
@@ -90,6 +90,25 @@ namespace gzk
         const bool special = same_x && !p_infinity && !q_infinity;
         if (__any_sync(0xffffffffu, special)) sum = select_fp(special, quad_add_special(p, q), sum);
         return select_fp(q_infinity, p, select_fp(p_infinity, q, sum));
+    }
+
+    // 2 p; called by whole warps.  (The curve has no point of order two, and ZZ = 0 stays ZZ = 0.)
+    __device__ __forceinline__ Fp quad_double(const Fp& p)
+    {
+        const int lane = threadIdx.x & 31, quad = lane & ~3, role = lane & 3;
+        // layer 1: X^2 | V = U^2 with U = 2 Y
+        const Fp twice = add(p, p);
+        const Fp s = quad_mul(role == 1 ? twice : p, role == 1 ? twice : p);
+        // layer 2: S = X V | W = U V | ZZ V | M^2 with M = 3 X^2
+        const Fp v = shfl_fp(s, quad + 1), xx = shfl_fp(s, quad);
+        const Fp m = add(add(xx, xx), xx);
+        const Fp t = quad_mul(role == 0 ? p : role == 1 ? twice : role == 2 ? p : m, role == 3 ? m : v);
+        // layer 3: M (S - X3) | W Y | - | W ZZZ, with X3 = M^2 - 2 S
+        const Fp sx = shfl_fp(t, quad), mm = shfl_fp(t, quad + 3), w = shfl_fp(t, quad + 1);
+        const Fp x3 = sub(mm, add(sx, sx));
+        const Fp f = quad_mul(role == 0 ? m : p, role == 0 ? sub(sx, x3) : w);
+        const Fp first = shfl_fp(f, quad);
+        return role == 0 ? x3 : role == 1 ? sub(first, f) : role == 2 ? t : f;
     }
 
     // x (lane 0) and y (lane 1) of the affine point, Montgomery; (0, 0) for the point at infinity.  All quads of the

@@ -5,15 +5,17 @@
 //                 bucket the number of hits is counted
 //   2. offsets    exclusive scan of the bucket counts (one CTA)
 //   3. scatter    (point index, sign) pairs are written bucket by bucket
-//   4. buckets    one thread per bucket adds its points (mixed XYZZ additions)
+//   4. buckets    one to eight lanes per bucket, longest buckets first, add its points (mixed XYZZ additions)
 //   5. bits       sum_d d*B_d of a bucket set: row and column sums of the buckets laid out as a
 //                 matrix, then the two small weighted sums split by the bits of the multiplier
-//   6. finish     per window Horner over the bits, shift by 2^(c*w), sum, to affine
+//   6. windows    sum of 2^b times the sums of the bits, a quad of lanes per bit; the host shifts the window
+//                 sums by 2^(c*w), adds them and converts to affine (254 dependent doublings: 0.2 ms there,
+//                 1.8 ms as a chain of one GPU thread)
 //
 // With a precomputed table of the points shifted by every window (gzk_msm_precompute:
 // 2^(c*w) P_i for all w, the layout for a resident SRS) the digits of all windows fall
 // into ONE set of 2^(c-1) buckets: no per-window reduction and no chain of c*w doublings
-// at the end (254 dependent doublings cost 2.8 ms whatever the size), and the window can
+// at the end, and the window can
 // be wider because only one window's buckets are reduced.
 //
 // Signed digits halve the bucket count (2^(c-1) per window): a negative digit adds
@@ -21,9 +23,12 @@
 // atomics of steps 1 and 3 leave the result bit-identical from run to run.
 #include <cstdlib>
 #include <cstring>
+#include <vector>
 
 #include "block.cuh"
 #include "g1.cuh"
+#include "g1_quad.cuh"
+#include "host_g1.hpp"
 
 namespace gzk
 {
@@ -32,10 +37,17 @@ namespace gzk
         constexpr int kThreads = 128;
         constexpr int kMaxWindows = 32;
         // Buckets with more entries than kBigBucket (skewed scalars: small integers, constant
-        // columns, the short top window) are cut into slices of kSliceEntries entries; one CTA
-        // sums a slice, one thread then adds the slices of a bucket.
+        // columns, the short top window) are cut into slices; one CTA sums a slice, one CTA then adds the
+        // slices of a bucket.  Short slices make the chains short (a thread adds four points of a slice of
+        // 512, and a quad of lanes joins them), and a very long bucket has at most 256.
         constexpr uint32_t kBigBucket = 1024;
-        constexpr uint32_t kSliceEntries = 2048;
+        constexpr uint32_t kSliceEntries = 512;
+        constexpr uint32_t kMaxSlices = 256;
+        __device__ __forceinline__ uint32_t slice_entries(uint32_t size)
+        {
+            const uint32_t even = (size + kMaxSlices - 1) / kMaxSlices;
+            return even > kSliceEntries ? even : kSliceEntries;
+        }
 
         struct BigItem
         {
@@ -96,19 +108,25 @@ namespace gzk
             }
         }
 
-        // exclusive scan of `count` uint32 values by one CTA (in place); also zeroes `cursor`
-        __global__ void __launch_bounds__(1024) msm_offsets_kernel(uint32_t* values, uint32_t* cursor, uint32_t count)
+        // start = exclusive scan of `count` sizes by one CTA; also zeroes `cursor`.  Eight values per thread and round:
+        // the rounds follow one another, and with one value each the 2^16 buckets of a table took 71 us.
+        constexpr uint32_t kScanElems = 8;
+        __global__ void __launch_bounds__(1024) msm_offsets_kernel(const uint32_t* sizes, uint32_t* start, uint32_t* cursor, uint32_t count)
         {
             __shared__ uint32_t warp_totals[32];
-            __shared__ uint32_t carry_in;
             const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-            if (threadIdx.x == 0) carry_in = 0;
-            __syncthreads();
-            for (uint32_t base = 0; base < count; base += 1024)
+            uint32_t carry = 0;
+            for (uint32_t base = 0; base < count; base += 1024 * kScanElems)
             {
-                const uint32_t idx = base + threadIdx.x;
-                const uint32_t v = idx < count ? values[idx] : 0;
-                uint32_t incl = v;
+                const uint32_t first = base + threadIdx.x * kScanElems;
+                uint32_t v[kScanElems], sum = 0;
+#pragma unroll
+                for (uint32_t j = 0; j < kScanElems; ++j)
+                {
+                    v[j] = first + j < count ? sizes[first + j] : 0;
+                    sum += v[j];
+                }
+                uint32_t incl = sum;
 #pragma unroll
                 for (int offset = 1; offset < 32; offset <<= 1)
                 {
@@ -117,18 +135,83 @@ namespace gzk
                 }
                 if (lane == 31) warp_totals[warp] = incl;
                 __syncthreads();
-                uint32_t warp_offset = 0;
-                for (uint32_t w2 = 0; w2 < warp; ++w2) warp_offset += warp_totals[w2];
-                const uint32_t start = carry_in;
-                if (idx < count)
+                uint32_t totals = warp_totals[lane];
+#pragma unroll
+                for (int offset = 1; offset < 32; offset <<= 1)
                 {
-                    values[idx] = start + warp_offset + incl - v;
-                    cursor[idx] = 0;
+                    const uint32_t up = __shfl_up_sync(0xffffffffu, totals, offset);
+                    if (lane >= static_cast<uint32_t>(offset)) totals += up;
                 }
-                __syncthreads();
-                if (threadIdx.x == 1023) carry_in = start + warp_offset + incl;
+                const uint32_t before = __shfl_sync(0xffffffffu, totals, (warp + 31) & 31);
+                uint32_t run = carry + (warp == 0 ? 0 : before) + incl - sum;
+#pragma unroll
+                for (uint32_t j = 0; j < kScanElems; ++j)
+                {
+                    if (first + j < count)
+                    {
+                        start[first + j] = run;
+                        cursor[first + j] = 0;
+                    }
+                    run += v[j];
+                }
+                carry += __shfl_sync(0xffffffffu, totals, 31);
                 __syncthreads();
             }
+        }
+
+        // The buckets by size, longest first: the lanes of a warp then add equally many points (bucket sizes scatter
+        // by their square root, so that the longest of 32 holds a fifth more than the mean at 240 points and two
+        // thirds more at 16), and the last warps to start have the least to do.  Buckets the slices take come last,
+        // with size 0.
+        constexpr uint32_t kSizeBins = kBigBucket + 1;
+        __device__ __forceinline__ uint32_t size_bin(uint32_t size) { return size > kBigBucket ? kBigBucket : kBigBucket - size; }
+        __global__ void __launch_bounds__(1024) msm_size_histogram_kernel(const uint32_t* bucket_size, uint32_t buckets, uint32_t* histogram)
+        {
+            __shared__ uint32_t local[kSizeBins];
+            for (uint32_t i = threadIdx.x; i < kSizeBins; i += blockDim.x) local[i] = 0;
+            __syncthreads();
+            const uint32_t b = blockIdx.x * blockDim.x + threadIdx.x;
+            if (b < buckets) atomicAdd(local + size_bin(bucket_size[b]), 1u);
+            __syncthreads();
+            for (uint32_t i = threadIdx.x; i < kSizeBins; i += blockDim.x)
+                if (local[i] != 0) atomicAdd(histogram + i, local[i]);
+        }
+        // `cursor`: one zeroed word per bin
+        __global__ void __launch_bounds__(1024) msm_order_kernel(const uint32_t* bucket_size, uint32_t buckets, const uint32_t* histogram, uint32_t* cursor, uint32_t* order)
+        {
+            __shared__ uint32_t first[kSizeBins], local[kSizeBins];
+            __shared__ uint32_t warp_totals[32];
+            static_assert(kSizeBins == 1025, "one bin per thread, the last one at the end");
+            const uint32_t t = threadIdx.x, lane = t & 31, warp = t >> 5;
+            const uint32_t v = histogram[t];
+            uint32_t incl = v;
+#pragma unroll
+            for (int offset = 1; offset < 32; offset <<= 1)
+            {
+                const uint32_t up = __shfl_up_sync(0xffffffffu, incl, offset);
+                if (lane >= static_cast<uint32_t>(offset)) incl += up;
+            }
+            if (lane == 31) warp_totals[warp] = incl;
+            local[t] = 0;
+            if (t == 0) local[1024] = 0;
+            __syncthreads();
+            uint32_t before = 0;
+            for (uint32_t w = 0; w < warp; ++w) before += warp_totals[w];
+            first[t] = before + incl - v;
+            if (t == 1023) first[1024] = before + incl;
+            __syncthreads();
+            const uint32_t b = blockIdx.x * blockDim.x + t;
+            uint32_t bin = 0, rank = 0;
+            if (b < buckets)
+            {
+                bin = size_bin(bucket_size[b]);
+                rank = atomicAdd(local + bin, 1u);
+            }
+            __syncthreads();
+            for (uint32_t i = t; i < kSizeBins; i += 1024)
+                if (local[i] != 0) first[i] += atomicAdd(cursor + i, local[i]);
+            __syncthreads();
+            if (b < buckets) order[first[bin] + rank] = b;
         }
 
         __global__ void __launch_bounds__(kThreads) msm_scatter_kernel(const uint32_t* code, uint64_t n, MsmPlan plan,
@@ -149,22 +232,49 @@ namespace gzk
             }
         }
 
+        template <int WIDTH>
+        __device__ __forceinline__ G1Xyzz shfl_down_xyzz(const G1Xyzz& p, int offset)
+        {
+            G1Xyzz o;
+#pragma unroll
+            for (int i = 0; i < FpCfg::N; ++i)
+            {
+                o.X.l[i] = __shfl_down_sync(0xffffffffu, p.X.l[i], offset, WIDTH);
+                o.Y.l[i] = __shfl_down_sync(0xffffffffu, p.Y.l[i], offset, WIDTH);
+                o.ZZ.l[i] = __shfl_down_sync(0xffffffffu, p.ZZ.l[i], offset, WIDTH);
+                o.ZZZ.l[i] = __shfl_down_sync(0xffffffffu, p.ZZZ.l[i], offset, WIDTH);
+            }
+            return o;
+        }
+
+        // LANES adjacent lanes per bucket, buckets in the order of their sizes
+        template <int LANES>
         __global__ void __launch_bounds__(kThreads) msm_buckets_kernel(const G1Affine* points, const uint32_t* bucket_start,
-                                                                      const uint32_t* bucket_size, const uint32_t* entries,
+                                                                      const uint32_t* bucket_size, const uint32_t* order, const uint32_t* entries,
                                                                       uint32_t buckets, G1Xyzz* out)
         {
-            const uint32_t b = blockIdx.x * blockDim.x + threadIdx.x;
-            if (b >= buckets) return;
-            const uint32_t start = bucket_start[b], size = bucket_size[b];
-            if (size > kBigBucket) return;  // handled cooperatively by msm_big_slices_kernel
+            const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
+            const uint32_t slot = t / LANES, part = t % LANES;
+            const uint32_t b = slot < buckets ? order[slot] : 0;
+            const uint32_t start = bucket_start[b], size = slot < buckets ? bucket_size[b] : 0;
+            const bool mine = size <= kBigBucket;  // longer ones are handled cooperatively by msm_big_slices_kernel
             G1Xyzz acc = G1Xyzz::infinity();
-#pragma unroll 1
-            for (uint32_t k = 0; k < size; ++k)
+            if (mine)
             {
-                const uint32_t e = entries[start + k];
-                acc = g1_add_mixed(acc, load_affine(points + (e >> 1)), (e & 1u) != 0);
+#pragma unroll 1
+                for (uint32_t k = part; k < size; k += LANES)
+                {
+                    const uint32_t e = entries[start + k];
+                    acc = g1_add_mixed(acc, load_affine(points + (e >> 1)), (e & 1u) != 0);
+                }
             }
-            store_xyzz(out + b, acc);
+#pragma unroll 1
+            for (int offset = LANES / 2; offset > 0; offset >>= 1)
+            {
+                const G1Xyzz other = shfl_down_xyzz<LANES>(acc, offset);
+                if (part < static_cast<uint32_t>(offset)) acc = g1_add(acc, other);
+            }
+            if (mine && part == 0 && slot < buckets) store_xyzz(out + b, acc);
         }
 
         // counters[0] = number of slice items, counters[1] = number of big buckets
@@ -175,7 +285,7 @@ namespace gzk
             if (b >= buckets) return;
             const uint32_t size = bucket_size[b];
             if (size <= kBigBucket) return;
-            const uint32_t slices = (size + kSliceEntries - 1) / kSliceEntries;
+            const uint32_t entries = slice_entries(size), slices = (size + entries - 1) / entries;
             const uint32_t first = atomicAdd(counters, slices);
             const uint32_t slot = atomicAdd(counters + 1, 1u);
             BigBucket bb;
@@ -192,83 +302,79 @@ namespace gzk
             }
         }
 
-        // CTA per slice item: the threads stride over the slice, then a shared-memory tree
+        // Sum over the 32 quads of a CTA of 128 threads, returned to quad 0
+        __device__ __forceinline__ Fp quad_cta_sum(Fp p, Fp* slots /* 16 */)
+        {
+            static_assert(kThreads == 128, "four warps of eight quads");
+#pragma unroll 1
+            for (int mask = 4; mask <= 64; mask <<= 1)
+            {
+                if (mask == 32)
+                {
+                    if ((threadIdx.x & 31) < 4) slots[(threadIdx.x >> 5) * 4 + (threadIdx.x & 3)] = p;
+                    __syncthreads();
+                    p = slots[threadIdx.x & 15];
+                }
+                p = quad_add(p, shfl_xor_fp(p, mask < 32 ? mask : mask >> 3));
+            }
+            return p;
+        }
+        // Slice items dealt to the CTAs: the threads stride over a slice, then the quads add the threads' sums up
+        // (four multiplications deep per addition: 258 -> 72 of them in sequence for a slice)
         __global__ void __launch_bounds__(kThreads) msm_big_slices_kernel(const G1Affine* points, const uint32_t* bucket_start,
                                                                          const uint32_t* bucket_size, const uint32_t* entries,
                                                                          const uint32_t* counters, const BigItem* items, G1Xyzz* partial)
         {
-            __shared__ G1Xyzz slots[kThreads];
-            if (blockIdx.x >= counters[0]) return;
-            const BigItem it = items[blockIdx.x];
-            const uint32_t start = bucket_start[it.bucket], size = bucket_size[it.bucket];
-            const uint32_t begin = it.slice * kSliceEntries;
-            const uint32_t end = begin + kSliceEntries < size ? begin + kSliceEntries : size;
-            G1Xyzz acc = G1Xyzz::infinity();
+            __shared__ G1Xyzz sums[kThreads];
+            __shared__ Fp slots[16];
+            const uint32_t quad = threadIdx.x >> 2, role = threadIdx.x & 3, count = counters[0];
+            for (uint32_t item = blockIdx.x; item < count; item += gridDim.x)
+            {
+                const BigItem it = items[item];
+                const uint32_t start = bucket_start[it.bucket], size = bucket_size[it.bucket], length = slice_entries(size);
+                const uint32_t begin = it.slice * length;
+                const uint32_t end = begin + length < size ? begin + length : size;
+                G1Xyzz acc = G1Xyzz::infinity();
 #pragma unroll 1
-            for (uint32_t k = begin + threadIdx.x; k < end; k += kThreads)
-            {
-                const uint32_t e = entries[start + k];
-                acc = g1_add_mixed(acc, load_affine(points + (e >> 1)), (e & 1u) != 0);
-            }
-            slots[threadIdx.x] = acc;
-            __syncthreads();
-            for (uint32_t offset = kThreads / 2; offset > 0; offset >>= 1)
-            {
-                if (threadIdx.x < offset) slots[threadIdx.x] = g1_add(slots[threadIdx.x], slots[threadIdx.x + offset]);
+                for (uint32_t k = begin + threadIdx.x; k < end; k += kThreads)
+                {
+                    const uint32_t e = entries[start + k];
+                    acc = g1_add_mixed(acc, load_affine(points + (e >> 1)), (e & 1u) != 0);
+                }
+                sums[threadIdx.x] = acc;
+                __syncthreads();
+                const Fp* parts = reinterpret_cast<const Fp*>(sums);
+                Fp p = parts[4 * quad + role];
+#pragma unroll 1
+                for (uint32_t j = 1; j < 4; ++j) p = quad_add(p, parts[4 * (quad + 32 * j) + role]);
+                p = quad_cta_sum(p, slots);
+                if (threadIdx.x < 4) store_fp(reinterpret_cast<Fp*>(partial + item) + role, p);
                 __syncthreads();
             }
-            if (threadIdx.x == 0) store_xyzz(partial + blockIdx.x, slots[0]);
         }
 
-        // CTA per big bucket: the threads stride over its slice partials, then a tree
+        // CTA per big bucket: the quads stride over its slice sums, then a tree
         __global__ void __launch_bounds__(kThreads) msm_big_combine_kernel(const uint32_t* counters, const BigBucket* big, const G1Xyzz* partial,
                                                                           G1Xyzz* out)
         {
-            __shared__ G1Xyzz slots[kThreads];
-            if (blockIdx.x >= counters[1]) return;
-            const BigBucket bb = big[blockIdx.x];
-            G1Xyzz acc = G1Xyzz::infinity();
-            for (uint32_t j = threadIdx.x; j < bb.slices; j += kThreads) acc = g1_add(acc, load_xyzz(partial + bb.first_item + j));
-            slots[threadIdx.x] = acc;
-            __syncthreads();
-            for (uint32_t offset = kThreads / 2; offset > 0; offset >>= 1)
+            __shared__ Fp slots[16];
+            const uint32_t quad = threadIdx.x >> 2, role = threadIdx.x & 3, count = counters[1];
+            for (uint32_t item = blockIdx.x; item < count; item += gridDim.x)
             {
-                if (threadIdx.x < offset) slots[threadIdx.x] = g1_add(slots[threadIdx.x], slots[threadIdx.x + offset]);
-                __syncthreads();
-            }
-            if (threadIdx.x == 0) store_xyzz(out + bb.bucket, slots[0]);
-        }
-
-        // one thread per window, then a tree over the windows; thread 0 converts to affine
-        __global__ void __launch_bounds__(kMaxWindows) msm_finish_kernel(const G1Xyzz* bit_sums, MsmPlan plan, G1Xyzz* out_xyzz,
-                                                                        G1Affine* out_canonical)
-        {
-            __shared__ G1Xyzz slots[kMaxWindows];
-            const uint32_t w = threadIdx.x;
-            G1Xyzz acc = G1Xyzz::infinity();
-            if (w < plan.windows)
-            {
-                for (int bit = static_cast<int>(plan.c) - 1; bit >= 0; --bit)
+                const BigBucket bb = big[item];
+                const Fp* parts = reinterpret_cast<const Fp*>(partial + bb.first_item);
+                Fp p = Fp::zero();
+#pragma unroll 1
+                for (uint32_t base = 0; base < bb.slices; base += kThreads / 4)
                 {
-                    acc = g1_double(acc);
-                    acc = g1_add(acc, load_xyzz(bit_sums + w * plan.c + bit));
+                    const uint32_t j = base + quad;
+                    Fp q = Fp::zero();
+                    if (j < bb.slices) q = parts[4 * static_cast<size_t>(j) + role];
+                    p = base == 0 ? q : quad_add(p, q);
                 }
-                for (uint32_t k = 0; k < w * plan.c; ++k) acc = g1_double(acc);
-            }
-            slots[w] = acc;
-            __syncthreads();
-            for (uint32_t offset = kMaxWindows / 2; offset > 0; offset >>= 1)
-            {
-                if (w < offset) slots[w] = g1_add(slots[w], slots[w + offset]);
+                p = quad_cta_sum(p, slots);
+                if (threadIdx.x < 4) store_fp(reinterpret_cast<Fp*>(out + bb.bucket) + role, p);
                 __syncthreads();
-            }
-            if (w == 0)
-            {
-                store_xyzz(out_xyzz, slots[0]);
-                G1Affine a = g1_to_affine(slots[0]);
-                a.x = from_mont(a.x);
-                a.y = from_mont(a.y);
-                store_affine(out_canonical, a);
             }
         }
 
@@ -280,90 +386,73 @@ namespace gzk
         // two weighted sums run over 2^h and 2^(c-1-h)+1 points only; those are split by the bits
         // of the multiplier: bit_sums[b] for b < h from the columns, for b >= h from the rows,
         // and sum_b 2^b * bit_sums[b] is the result.
-        __device__ __forceinline__ G1Xyzz cta_tree_sum(G1Xyzz acc, G1Xyzz* slots)
-        {
-            slots[threadIdx.x] = acc;
-            __syncthreads();
-            for (uint32_t offset = kThreads / 2; offset > 0; offset >>= 1)
-            {
-                if (threadIdx.x < offset) slots[threadIdx.x] = g1_add(slots[threadIdx.x], slots[threadIdx.x + offset]);
-                __syncthreads();
-            }
-            return slots[0];
-        }
-        // CTAs [0, rows): row sums; CTAs [rows, rows + cols): column sums.  rc = [rows row sums][cols column sums]
-        // (blockIdx.y = window when every window has its own bucket set)
+        // LANES adjacent lanes per line: lines [0, rows) are rows, lines [rows, rows + cols) columns.  rc = [rows row
+        // sums][cols column sums] (blockIdx.y = window when every window has its own bucket set)
+        template <int LANES>
         __global__ void __launch_bounds__(kThreads) msm_rowcol_kernel(const G1Xyzz* buckets, uint32_t half, uint32_t h, uint32_t rows, G1Xyzz* rc)
         {
-            __shared__ G1Xyzz slots[kThreads];
-            const uint32_t cols = 1u << h;
+            const uint32_t cols = 1u << h, t = blockIdx.x * kThreads + threadIdx.x, line = t / LANES, part = t % LANES;
             buckets += static_cast<uint64_t>(blockIdx.y) * half;
             rc += static_cast<uint64_t>(blockIdx.y) * (rows + cols);
+            // d = first + k * step for k < length, of which 1 .. half are buckets
+            const bool row = line < rows;
+            const uint32_t first = row ? line << h : line - rows, step = row ? 1u : cols, length = line >= rows + cols ? 0u : row ? cols : rows;
             G1Xyzz acc = G1Xyzz::infinity();
-            if (blockIdx.x < rows)
+#pragma unroll 1
+            for (uint32_t k = part; k < length; k += LANES)
             {
-                const uint32_t hi = blockIdx.x;
-                for (uint32_t lo = threadIdx.x; lo < cols; lo += kThreads)
-                {
-                    const uint32_t d = (hi << h) | lo;
-                    if (d >= 1 && d <= half) acc = g1_add(acc, load_xyzz(buckets + (d - 1)));
-                }
+                const uint32_t d = first + k * step;
+                if (d >= 1 && d <= half) acc = g1_add(acc, load_xyzz(buckets + (d - 1)));
             }
-            else
+#pragma unroll 1
+            for (int offset = LANES / 2; offset > 0; offset >>= 1)
             {
-                const uint32_t lo = blockIdx.x - rows;
-                for (uint32_t hi = threadIdx.x; hi < rows; hi += kThreads)
-                {
-                    const uint32_t d = (hi << h) | lo;
-                    if (d >= 1 && d <= half) acc = g1_add(acc, load_xyzz(buckets + (d - 1)));
-                }
+                const G1Xyzz other = shfl_down_xyzz<LANES>(acc, offset);
+                if (part < static_cast<uint32_t>(offset)) acc = g1_add(acc, other);
             }
-            const G1Xyzz total = cta_tree_sum(acc, slots);
-            if (threadIdx.x == 0) store_xyzz(rc + blockIdx.x, total);
+            if (part == 0 && line < rows + cols) store_xyzz(rc + line, acc);
         }
+
         // CTA b < h: sum of the column sums whose lo has bit b; CTA b >= h: sum of the row sums whose hi has bit b - h
         __global__ void __launch_bounds__(kThreads) msm_rowcol_bits_kernel(const G1Xyzz* rc, uint32_t h, uint32_t rows, G1Xyzz* bit_sums)
         {
-            __shared__ G1Xyzz slots[kThreads];
-            const uint32_t b = blockIdx.x;
+            __shared__ Fp slots[16];
+            const uint32_t b = blockIdx.x, quad = threadIdx.x >> 2, role = threadIdx.x & 3;
             rc += static_cast<uint64_t>(blockIdx.y) * (rows + (1u << h));
             bit_sums += static_cast<uint64_t>(blockIdx.y) * gridDim.x;
             const bool from_cols = b < h;
             const uint32_t count = from_cols ? (1u << h) : rows;
             const uint32_t bit = from_cols ? b : b - h;
-            const G1Xyzz* src = from_cols ? rc + rows : rc;
-            G1Xyzz acc = G1Xyzz::infinity();
-            for (uint32_t j = threadIdx.x; j < count; j += kThreads)
-                if ((j >> bit) & 1u) acc = g1_add(acc, load_xyzz(src + j));
-            const G1Xyzz total = cta_tree_sum(acc, slots);
-            if (threadIdx.x == 0) store_xyzz(bit_sums + b, total);
+            const Fp* src = reinterpret_cast<const Fp*>(from_cols ? rc + rows : rc);
+            Fp acc = Fp::zero();
+#pragma unroll 1
+            for (uint32_t base = 0; base < (count + 1) / 2; base += kThreads / 4)
+            {
+                const uint32_t i = base + quad;  // the i-th number with that bit set
+                const uint32_t j = (i >> bit) << (bit + 1) | 1u << bit | (i & ((1u << bit) - 1u));
+                Fp p = Fp::zero();
+                if (j < count) p = src[4 * static_cast<size_t>(j) + role];
+                acc = base == 0 ? p : quad_add(acc, p);
+            }
+            acc = quad_cta_sum(acc, slots);
+            if (threadIdx.x < 4) store_fp(reinterpret_cast<Fp*>(bit_sums + b) + role, acc);
         }
-        // thread b shifts the sum of bit b by b doublings (at most c - 1), then a tree; thread 0 converts to affine
-        __global__ void __launch_bounds__(kMaxWindows) msm_finish_shared_kernel(const G1Xyzz* bit_sums, uint32_t c, G1Xyzz* out_xyzz, G1Affine* out_canonical)
+        // CTA per bucket set: quad b doubles the sum of bit b by b times, then a tree
+        __global__ void __launch_bounds__(kThreads) msm_window_sums_kernel(const G1Xyzz* bit_sums, uint32_t c, G1Xyzz* out)
         {
-            __shared__ G1Xyzz slots[kMaxWindows];
-            const uint32_t b = threadIdx.x;
-            G1Xyzz acc = G1Xyzz::infinity();
-            if (b < c)
+            __shared__ Fp slots[16];
+            const uint32_t b = threadIdx.x >> 2, role = threadIdx.x & 3;
+            bit_sums += static_cast<uint64_t>(blockIdx.x) * c;
+            Fp p = Fp::zero();
+            if (b < c) p = reinterpret_cast<const Fp*>(bit_sums)[4 * b + role];
+#pragma unroll 1
+            for (uint32_t k = 0; k + 1 < c; ++k)
             {
-                acc = load_xyzz(bit_sums + b);
-                for (uint32_t k = 0; k < b; ++k) acc = g1_double(acc);
+                const Fp twice = quad_double(p);
+                if (k < b) p = twice;
             }
-            slots[b] = acc;
-            __syncthreads();
-            for (uint32_t offset = kMaxWindows / 2; offset > 0; offset >>= 1)
-            {
-                if (b < offset) slots[b] = g1_add(slots[b], slots[b + offset]);
-                __syncthreads();
-            }
-            if (b == 0)
-            {
-                store_xyzz(out_xyzz, slots[0]);
-                G1Affine a = g1_to_affine(slots[0]);
-                a.x = from_mont(a.x);
-                a.y = from_mont(a.y);
-                store_affine(out_canonical, a);
-            }
+            p = quad_cta_sum(p, slots);
+            if (threadIdx.x < 4) store_fp(reinterpret_cast<Fp*>(out + blockIdx.x) + role, p);
         }
 
         // next[i] = 2^c * prev[i] (affine Montgomery in and out; one inversion per point, all in parallel)
@@ -415,18 +504,47 @@ namespace gzk
             return p;
         }
 
+        // Window of a plan with a bucket set per window, by multiplications: ten per point and window, about 45 per
+        // bucket for its two additions in the row and column sums, and half a window again where the top window has
+        // so few bits that its handful of buckets goes through the slices.
+        int plan_window_bits(uint64_t n)
+        {
+            int best = 8;
+            double best_cost = 0.0;
+            for (int c = 8; c <= 16; ++c)
+            {
+                const int windows = (256 + c - 1) / c, top_bits = 255 - c * (windows - 1);
+                double cost = 10.0 * static_cast<double>(n) * windows + 45.0 * windows * static_cast<double>(1u << (c - 1));
+                if (static_cast<double>(n) > static_cast<double>(kBigBucket) * static_cast<double>(1u << top_bits)) cost += 5.0 * static_cast<double>(n);
+                if (best_cost == 0.0 || cost < best_cost)
+                {
+                    best_cost = cost;
+                    best = c;
+                }
+            }
+            return best;
+        }
+
+        // Lanes per bucket: as many as leave eight warps for every scheduler and two points for every lane.  One lane
+        // per bucket left 13312 lanes for 2^16 points: bucket pass 1773 us, with window and lanes chosen as here 662 us
+        // (whole call 5.27 -> 1.37 ms); 2^20 points on their table, 240 to a bucket: 7.93 -> 6.89 ms (call 9.36 -> 7.75 ms).
+        uint32_t bucket_lanes(const gzk_ctx* ctx, uint64_t buckets, uint64_t entries)
+        {
+            const uint64_t threads = static_cast<uint64_t>(ctx->sm_count) * 4 * 8 * 32;
+            uint32_t lanes = 1;
+            while (lanes < 8 && buckets * lanes * 2 <= threads && entries >= buckets * lanes * 4) lanes *= 2;
+#ifdef GZK_BUILD_TUNING
+            if (const char* forced = std::getenv("GZK_MSM_LANES")) lanes = static_cast<uint32_t>(std::atoi(forced));
+#endif
+            return lanes;
+        }
+
         MsmPlan make_plan(uint64_t n)
         {
-            uint32_t log2n = 0;
-            while ((1ULL << (log2n + 1)) <= n) ++log2n;
-            // larger windows mean fewer mixed additions (n per window) but 2^(c-1) * c / 2 full
-            // additions per window in the bit-split reduction; log2(n) - 7 balances the two
-            int c = static_cast<int>(log2n) - 6;
+            int c = plan_window_bits(n);
 #ifdef GZK_BUILD_TUNING
             if (const char* forced = std::getenv("GZK_MSM_WINDOW")) c = std::atoi(forced);
 #endif
-            if (c < 8) c = 8;
-            if (c > 16) c = 16;
             MsmPlan p;
             p.c = static_cast<uint32_t>(c);
             p.windows = (256 + p.c - 1) / p.c;
@@ -436,9 +554,7 @@ namespace gzk
         }
     }
 
-    // MSM over device-resident scalars and points; the XYZZ result is left in
-    // `out_xyzz` (device, optional use by multi-GPU combiners) and the canonical
-    // affine result is copied to `out_host`.
+    // MSM over device-resident scalars and points; the canonical affine result is written to `out_host`.
     static int msm_run_plan(gzk_ctx* ctx, const gzk_buf* scalars, const gzk_buf* points, uint64_t n, const MsmPlan& plan, uint8_t out_host[96])
     {
         const uint64_t buckets = plan.shared ? plan.half : static_cast<uint64_t>(plan.windows) * plan.half;
@@ -453,7 +569,7 @@ namespace gzk
         const uint32_t bucket_sets = plan.shared ? 1u : plan.windows;
         const size_t chunk_bytes = static_cast<size_t>(bucket_sets) * (static_cast<size_t>(split_rows) + (1u << split_h)) * sizeof(G1Xyzz);
         const size_t total = big_bytes + 2 * code_bytes + 3 * bucket_u32 + buckets * sizeof(G1Xyzz) + static_cast<size_t>(plan.windows) * plan.c * sizeof(G1Xyzz) +
-                             chunk_bytes + sizeof(G1Xyzz) + sizeof(G1Affine) + 8192;
+                             chunk_bytes + static_cast<size_t>(plan.windows) * sizeof(G1Xyzz) + bucket_u32 + 2 * kSizeBins * sizeof(uint32_t) + 8192;
         void* scratch = nullptr;
         int rc = ensure_scratch(ctx, 1, total, &scratch);
         if (rc != GZK_OK) return rc;
@@ -465,8 +581,9 @@ namespace gzk
         };
         G1Xyzz* bucket_points = reinterpret_cast<G1Xyzz*>(take(buckets * sizeof(G1Xyzz)));
         G1Xyzz* bit_sums = reinterpret_cast<G1Xyzz*>(take(static_cast<size_t>(plan.windows) * plan.c * sizeof(G1Xyzz)));
-        G1Xyzz* result_xyzz = reinterpret_cast<G1Xyzz*>(take(sizeof(G1Xyzz)));
-        G1Affine* result_affine = reinterpret_cast<G1Affine*>(take(sizeof(G1Affine)));
+        G1Xyzz* window_sums = reinterpret_cast<G1Xyzz*>(take(static_cast<size_t>(plan.windows) * sizeof(G1Xyzz)));
+        uint32_t* order = reinterpret_cast<uint32_t*>(take(bucket_u32));
+        uint32_t* size_bins = reinterpret_cast<uint32_t*>(take(2 * kSizeBins * sizeof(uint32_t)));
         uint32_t* code = reinterpret_cast<uint32_t*>(take(code_bytes));
         uint32_t* entries = reinterpret_cast<uint32_t*>(take(code_bytes));
         uint32_t* bucket_size = reinterpret_cast<uint32_t*>(take(bucket_u32));
@@ -489,10 +606,9 @@ namespace gzk
             msm_digits_kernel<<<static_cast<unsigned>((n + kThreads - 1) / kThreads), kThreads, 0, ctx->stream>>>(s, n, plan, code, bucket_size);
         }
         GZK_CUDA_TRY(ctx, cudaGetLastError());
-        GZK_CUDA_TRY(ctx, cudaMemcpyAsync(bucket_start, bucket_size, bucket_u32, cudaMemcpyDeviceToDevice, ctx->stream));
         {
             LaunchScope scope(ctx, "msm_offsets");
-            msm_offsets_kernel<<<1, 1024, 0, ctx->stream>>>(bucket_start, cursor, static_cast<uint32_t>(buckets));
+            msm_offsets_kernel<<<1, 1024, 0, ctx->stream>>>(bucket_size, bucket_start, cursor, static_cast<uint32_t>(buckets));
         }
         GZK_CUDA_TRY(ctx, cudaGetLastError());
         {
@@ -511,38 +627,50 @@ namespace gzk
                 bucket_size, static_cast<uint32_t>(buckets), big_counters, big_items, big_buckets);
         }
         GZK_CUDA_TRY(ctx, cudaGetLastError());
+        GZK_CUDA_TRY(ctx, cudaMemsetAsync(size_bins, 0, 2 * kSizeBins * sizeof(uint32_t), ctx->stream));
         {
-            LaunchScope scope(ctx, "msm_buckets");
-            msm_buckets_kernel<<<static_cast<unsigned>((buckets + kThreads - 1) / kThreads), kThreads, 0, ctx->stream>>>(
-                static_cast<const G1Affine*>(points->dptr), bucket_start, bucket_size, entries, static_cast<uint32_t>(buckets), bucket_points);
+            LaunchScope scope(ctx, "msm_order", 2);
+            const unsigned blocks = static_cast<unsigned>((buckets + 1023) / 1024);
+            msm_size_histogram_kernel<<<blocks, 1024, 0, ctx->stream>>>(bucket_size, static_cast<uint32_t>(buckets), size_bins);
+            msm_order_kernel<<<blocks, 1024, 0, ctx->stream>>>(bucket_size, static_cast<uint32_t>(buckets), size_bins, size_bins + kSizeBins, order);
         }
         GZK_CUDA_TRY(ctx, cudaGetLastError());
         {
-            // grids are upper bounds; CTAs beyond the counted work return at once
+            LaunchScope scope(ctx, "msm_buckets");
+            const uint32_t lanes = bucket_lanes(ctx, buckets, total_entries);
+            const auto kernel = lanes == 1 ? msm_buckets_kernel<1> : lanes == 2 ? msm_buckets_kernel<2> : lanes == 4 ? msm_buckets_kernel<4> : msm_buckets_kernel<8>;
+            kernel<<<static_cast<unsigned>((buckets * lanes + kThreads - 1) / kThreads), kThreads, 0, ctx->stream>>>(
+                static_cast<const G1Affine*>(points->dptr), bucket_start, bucket_size, order, entries, static_cast<uint32_t>(buckets), bucket_points);
+        }
+        GZK_CUDA_TRY(ctx, cudaGetLastError());
+        {
+            // the counts stay on the device: grids that fill the chip, or the upper bound where that is less
             LaunchScope scope(ctx, "msm_big_buckets", 2);
-            msm_big_slices_kernel<<<static_cast<unsigned>(max_items), kThreads, 0, ctx->stream>>>(
+            const uint64_t cap = static_cast<uint64_t>(ctx->sm_count) * 4;
+            msm_big_slices_kernel<<<static_cast<unsigned>(max_items < cap ? max_items : cap), kThreads, 0, ctx->stream>>>(
                 static_cast<const G1Affine*>(points->dptr), bucket_start, bucket_size, entries, big_counters, big_items, big_partial);
-            msm_big_combine_kernel<<<static_cast<unsigned>(max_big), kThreads, 0, ctx->stream>>>(
+            msm_big_combine_kernel<<<static_cast<unsigned>(max_big < cap ? max_big : cap), kThreads, 0, ctx->stream>>>(
                 big_counters, big_buckets, big_partial, bucket_points);
         }
         GZK_CUDA_TRY(ctx, cudaGetLastError());
         {
-            LaunchScope scope(ctx, "msm_bits", 2);
-            msm_rowcol_kernel<<<dim3(split_rows + (1u << split_h), bucket_sets), kThreads, 0, ctx->stream>>>(bucket_points, plan.half, split_h, split_rows,
-                                                                                                    bit_partial);
-            msm_rowcol_bits_kernel<<<dim3(plan.c, bucket_sets), kThreads, 0, ctx->stream>>>(bit_partial, split_h, split_rows, bit_sums);
-        }
-        GZK_CUDA_TRY(ctx, cudaGetLastError());
-        {
-            LaunchScope scope(ctx, "msm_finish");
-            if (plan.shared)
-                msm_finish_shared_kernel<<<1, kMaxWindows, 0, ctx->stream>>>(bit_sums, plan.c, result_xyzz, result_affine);
+            LaunchScope scope(ctx, "msm_bits", 3);
+            const uint32_t lines = split_rows + (1u << split_h);
+            // a line by one warp while that leaves the chip short of warps, else by eight lanes (32 lanes add five
+            // levels of a tree to each line: for one set of 2^16 buckets the shorter chain, for 26 sets the longer)
+            if (static_cast<uint64_t>(lines) * bucket_sets <= static_cast<uint64_t>(ctx->sm_count) * 8)
+                msm_rowcol_kernel<32><<<dim3((lines * 32 + kThreads - 1) / kThreads, bucket_sets), kThreads, 0, ctx->stream>>>(bucket_points, plan.half, split_h, split_rows, bit_partial);
             else
-                msm_finish_kernel<<<1, kMaxWindows, 0, ctx->stream>>>(bit_sums, plan, result_xyzz, result_affine);
+                msm_rowcol_kernel<8><<<dim3((lines * 8 + kThreads - 1) / kThreads, bucket_sets), kThreads, 0, ctx->stream>>>(bucket_points, plan.half, split_h, split_rows, bit_partial);
+            msm_rowcol_bits_kernel<<<dim3(plan.c, bucket_sets), kThreads, 0, ctx->stream>>>(bit_partial, split_h, split_rows, bit_sums);
+            msm_window_sums_kernel<<<bucket_sets, kThreads, 0, ctx->stream>>>(bit_sums, plan.c, window_sums);
         }
         GZK_CUDA_TRY(ctx, cudaGetLastError());
-        GZK_CUDA_TRY(ctx, cudaMemcpyAsync(out_host, result_affine, 96, cudaMemcpyDeviceToHost, ctx->stream));
+        // the shifts of the windows are one chain of c * w doublings: the host's part
+        HostXyzz sums[kMaxWindows];
+        GZK_CUDA_TRY(ctx, cudaMemcpyAsync(sums, window_sums, bucket_sets * sizeof(HostXyzz), cudaMemcpyDeviceToHost, ctx->stream));
         GZK_CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream));
+        host_to_affine_bytes(host_horner(sums, bucket_sets, plan.c), out_host);
         return GZK_OK;
     }
 }

@@ -178,3 +178,34 @@ def test_msm_precomputed_rejects_short_table(be):
     pts = be.g1_fixed_base_mul(G, be.upload(fr_array(list(range(1, n + 1))), KIND_FR), n)
     with pytest.raises(GzkError):
         be.msm_precomputed(be.upload(fr_array([1] * n), KIND_FR), pts, n, 16)  # a plain point buffer is not a table
+
+
+# (size, scalars): every number of lanes per bucket, both widths of the row and column sums, buckets that the slices
+# take and buckets just below them, windows whose top digits are few
+@pytest.mark.parametrize("n,kind", [(64, "random"), (1500, "random"), (4000, "random"), (20000, "random"), (70001, "random"), (4000, "constant"), (4000, "small"),
+                                    (4000, "zero"), (20000, "skewed")])
+def test_msm_plans(be, n, kind):
+    from project_b200 import KIND_FR
+
+    rng = random.Random(n)
+    ks = pyref.rand_fr(rng, n)
+    if kind == "random":
+        scalars = pyref.rand_fr(rng, n)
+    elif kind == "constant":
+        scalars = [pyref.rand_fr(rng, 1)[0]] * n
+    elif kind == "small":
+        scalars = [rng.randint(-100, 100) % R for _ in range(n)]
+    elif kind == "zero":
+        scalars = [0] * n
+    else:
+        scalars = [7 if i < 1024 else 9 if i < 2049 else 11 if i < 10000 else rng.randrange(R) for i in range(n)]
+    pts = be.g1_fixed_base_mul(G, be.upload(fr_array(ks), KIND_FR), n)
+    s = be.upload(fr_array(scalars), KIND_FR)
+    total = sum(k * v for k, v in zip(ks, scalars)) % R
+    want = pyref.g1_bytes(pyref.g1_mul(total, (pyref.GX, pyref.GY))) if total else bytes(96)
+    assert bytes(be.msm(s, pts, n)) == want
+    if n <= 4000:
+        for bits in (8, 13, 16, 20):
+            table, used = be.msm_precompute(pts, n, bits)
+            assert bytes(be.msm_precomputed(s, table, n, used)) == want
+            table.free()

@@ -52,3 +52,7 @@ def test_same_base_of_order_three(be):
 def test_weights_through_the_cta_inversion(be, log2n):
     x = fr_array([0x123456789ABCDEF0123456789 + log2n])[0]
     assert np.array_equal(be.bary_weights(log2n, x).download(), ora.bary_weights(x, 1 << log2n))
+
+
+def test_host_point_arithmetic():
+    _run(os.path.join(ROOT, "tests", "host", "host_g1_check.cpp"))
