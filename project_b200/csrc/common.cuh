@@ -90,6 +90,9 @@ struct gzk_ctx
     void* pinned = nullptr;  // small pinned staging area for results
     size_t pinned_bytes = 0;
     int* d_status = nullptr;  // device-side status word (zero-denominator flags etc.)
+    int* h_status = nullptr;  // pinned copy of it, read at the end of a call that waits
+    // zero between the kernels of the stream: counts the CTAs of a launch that have left their partial result
+    uint32_t* arrival_counter() const { return reinterpret_cast<uint32_t*>(d_status) + 8; }
     // pinned ring for the small uploads of deferred mode: the data is copied into a slot and the
     // call returns without waiting; a slot is reused once the copy that read it has completed
     static constexpr int kUploadSlots = 16;
@@ -139,6 +142,8 @@ namespace gzk
     // stream and turn a raised status word into an error; in deferred mode return at once
     // (the status word stays raised until gzk_ctx_synchronize reports it).
     int finish_call(gzk_ctx* ctx, const char* invalid_message);
+    // The same for a call whose kernels raise no status: nothing to read back.
+    int wait_call(gzk_ctx* ctx);
     // Clears the status word at the start of a call (not in deferred mode, where it is sticky).
     int begin_call(gzk_ctx* ctx);
 
@@ -146,6 +151,7 @@ namespace gzk
     Fr host_fr_from_bytes(const uint8_t* bytes, bool* canonical_ok);
     void host_fr_to_bytes(const Fr& canonical, uint8_t* bytes);
     Fr host_root_of_unity(unsigned log2n);  // Montgomery form
+    Fr host_fr_mul(const Fr& a, const Fr& b);  // Montgomery product on four 64-bit limbs
 
 #define GZK_CUDA_TRY(ctx, expr)                                         \
     do                                                                  \

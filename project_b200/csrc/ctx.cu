@@ -141,10 +141,16 @@ namespace gzk
     int finish_call(gzk_ctx* ctx, const char* invalid_message)
     {
         if (ctx->deferred) return GZK_OK;
-        int status[2] = {0, 0};
-        GZK_CUDA_TRY(ctx, cudaMemcpyAsync(status, ctx->d_status, sizeof(status), cudaMemcpyDeviceToHost, ctx->stream));
+        // into pinned memory: a copy to pageable memory goes through the runtime's staging area and waits twice
+        GZK_CUDA_TRY(ctx, cudaMemcpyAsync(ctx->h_status, ctx->d_status, 2 * sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
         GZK_CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream));
-        return status_to_error(ctx, status, invalid_message);
+        return status_to_error(ctx, ctx->h_status, invalid_message);
+    }
+
+    int wait_call(gzk_ctx* ctx)
+    {
+        if (!ctx->deferred) GZK_CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream));
+        return GZK_OK;
     }
 
     Fr host_fr_from_bytes(const uint8_t* bytes, bool* canonical_ok)
@@ -166,6 +172,98 @@ namespace gzk
     }
 
     void host_fr_to_bytes(const Fr& canonical, uint8_t* bytes) { std::memcpy(bytes, canonical.l, 32); }
+
+    namespace
+    {
+        // Montgomery product on four 64-bit limbs (coarsely integrated operand scanning): the host's
+        // 64x64->128 multiplier does in 32 products what the kernels' 32-bit limb code does in 128.
+        struct HostFr64
+        {
+            uint64_t modulus[4], r2[4], n0;  // n0 = -modulus^-1 mod 2^64
+            HostFr64()
+            {
+                const Fr rr = Fr::r2();
+                for (int i = 0; i < 4; ++i)
+                {
+                    modulus[i] = static_cast<uint64_t>(FrCfg::mod(2 * i)) | (static_cast<uint64_t>(FrCfg::mod(2 * i + 1)) << 32);
+                    r2[i] = static_cast<uint64_t>(rr.l[2 * i]) | (static_cast<uint64_t>(rr.l[2 * i + 1]) << 32);
+                }
+                uint64_t x = 1;  // Newton: x <- x (2 - m x) doubles the correct low bits
+                for (int i = 0; i < 6; ++i) x *= 2 - modulus[0] * x;
+                n0 = ~x + 1;
+            }
+            void mul(const uint64_t a[4], const uint64_t b[4], uint64_t out[4]) const
+            {
+                using u128 = unsigned __int128;
+                uint64_t t[6] = {0, 0, 0, 0, 0, 0};
+                for (int i = 0; i < 4; ++i)
+                {
+                    uint64_t carry = 0;
+                    for (int j = 0; j < 4; ++j)
+                    {
+                        const u128 w = static_cast<u128>(a[j]) * b[i] + t[j] + carry;
+                        t[j] = static_cast<uint64_t>(w);
+                        carry = static_cast<uint64_t>(w >> 64);
+                    }
+                    u128 top = static_cast<u128>(t[4]) + carry;
+                    t[4] = static_cast<uint64_t>(top);
+                    t[5] = static_cast<uint64_t>(top >> 64);
+                    const uint64_t q = t[0] * n0;
+                    u128 w = static_cast<u128>(q) * modulus[0] + t[0];
+                    carry = static_cast<uint64_t>(w >> 64);
+                    for (int j = 1; j < 4; ++j)
+                    {
+                        w = static_cast<u128>(q) * modulus[j] + t[j] + carry;
+                        t[j - 1] = static_cast<uint64_t>(w);
+                        carry = static_cast<uint64_t>(w >> 64);
+                    }
+                    top = static_cast<u128>(t[4]) + carry;
+                    t[3] = static_cast<uint64_t>(top);
+                    t[4] = t[5] + static_cast<uint64_t>(top >> 64);
+                }
+                // t < 2 * modulus: one conditional subtraction
+                uint64_t d[4];
+                unsigned __int128 borrow = 0;
+                for (int j = 0; j < 4; ++j)
+                {
+                    const u128 w = static_cast<u128>(t[j]) - modulus[j] - static_cast<uint64_t>(borrow);
+                    d[j] = static_cast<uint64_t>(w);
+                    borrow = (w >> 64) & 1;
+                }
+                const bool keep = t[4] == 0 && borrow != 0;
+                for (int j = 0; j < 4; ++j) out[j] = keep ? t[j] : d[j];
+            }
+        };
+        const HostFr64& host_fr64()
+        {
+            static const HostFr64 f;
+            return f;
+        }
+        // product of two canonical elements, canonical: (a R^2 / R) b / R
+        Fr host_mul_canonical(const Fr& a, const Fr& b)
+        {
+            const HostFr64& f = host_fr64();
+            uint64_t x[4], y[4], ar[4], out[4];
+            std::memcpy(x, a.l, 32);
+            std::memcpy(y, b.l, 32);
+            f.mul(x, f.r2, ar);
+            f.mul(ar, y, out);
+            Fr r;
+            std::memcpy(r.l, out, 32);
+            return r;
+        }
+    }
+
+    Fr host_fr_mul(const Fr& a, const Fr& b)
+    {
+        uint64_t x[4], y[4], out[4];
+        std::memcpy(x, a.l, 32);
+        std::memcpy(y, b.l, 32);
+        host_fr64().mul(x, y, out);
+        Fr r;
+        std::memcpy(r.l, out, 32);
+        return r;
+    }
 
     namespace
     {
@@ -308,6 +406,7 @@ extern "C"
             cudaEventCreateWithFlags(&ctx->copy_event, cudaEventDisableTiming) != cudaSuccess ||
             cudaEventCreateWithFlags(&ctx->order_event, cudaEventDisableTiming) != cudaSuccess ||
             cudaMalloc(reinterpret_cast<void**>(&ctx->d_status), 64) != cudaSuccess ||
+            cudaMallocHost(reinterpret_cast<void**>(&ctx->h_status), 64) != cudaSuccess ||
             // cleared ON THE CONTEXT'S STREAM and waited for: a cudaMemset would run on the legacy default stream, which
             // is not ordered with this non-blocking stream, so the first status read (gzk_ctx_set_deferred,
             // microseconds later) could overtake it and see whatever the memory held before - e.g. the
@@ -345,6 +444,7 @@ extern "C"
             for (auto e : ctx->upload_done) cudaEventDestroy(e);
         }
         if (ctx->d_status != nullptr) cudaFree(ctx->d_status);
+        if (ctx->h_status != nullptr) cudaFreeHost(ctx->h_status);
         timing_collect(ctx);
         g1_release_tables(ctx);
         for (auto e : ctx->event_pool) cudaEventDestroy(e);
@@ -674,82 +774,6 @@ extern "C"
         if (log2n > 32) return fail(ctx, GZK_E_INVALID, "domain size exceeds the 2-adicity of Fr");
         host_fr_to_bytes(from_mont(host_root_of_unity(log2n)), out);
         return GZK_OK;
-    }
-
-    namespace
-    {
-        // Montgomery product on four 64-bit limbs (coarsely integrated operand scanning): the host's
-        // 64x64->128 multiplier does in 32 products what the kernels' 32-bit limb code does in 128.
-        struct HostFr64
-        {
-            uint64_t modulus[4], r2[4], n0;  // n0 = -modulus^-1 mod 2^64
-            HostFr64()
-            {
-                const Fr rr = Fr::r2();
-                for (int i = 0; i < 4; ++i)
-                {
-                    modulus[i] = static_cast<uint64_t>(FrCfg::mod(2 * i)) | (static_cast<uint64_t>(FrCfg::mod(2 * i + 1)) << 32);
-                    r2[i] = static_cast<uint64_t>(rr.l[2 * i]) | (static_cast<uint64_t>(rr.l[2 * i + 1]) << 32);
-                }
-                uint64_t x = 1;  // Newton: x <- x (2 - m x) doubles the correct low bits
-                for (int i = 0; i < 6; ++i) x *= 2 - modulus[0] * x;
-                n0 = ~x + 1;
-            }
-            void mul(const uint64_t a[4], const uint64_t b[4], uint64_t out[4]) const
-            {
-                using u128 = unsigned __int128;
-                uint64_t t[6] = {0, 0, 0, 0, 0, 0};
-                for (int i = 0; i < 4; ++i)
-                {
-                    uint64_t carry = 0;
-                    for (int j = 0; j < 4; ++j)
-                    {
-                        const u128 w = static_cast<u128>(a[j]) * b[i] + t[j] + carry;
-                        t[j] = static_cast<uint64_t>(w);
-                        carry = static_cast<uint64_t>(w >> 64);
-                    }
-                    u128 top = static_cast<u128>(t[4]) + carry;
-                    t[4] = static_cast<uint64_t>(top);
-                    t[5] = static_cast<uint64_t>(top >> 64);
-                    const uint64_t q = t[0] * n0;
-                    u128 w = static_cast<u128>(q) * modulus[0] + t[0];
-                    carry = static_cast<uint64_t>(w >> 64);
-                    for (int j = 1; j < 4; ++j)
-                    {
-                        w = static_cast<u128>(q) * modulus[j] + t[j] + carry;
-                        t[j - 1] = static_cast<uint64_t>(w);
-                        carry = static_cast<uint64_t>(w >> 64);
-                    }
-                    top = static_cast<u128>(t[4]) + carry;
-                    t[3] = static_cast<uint64_t>(top);
-                    t[4] = t[5] + static_cast<uint64_t>(top >> 64);
-                }
-                // t < 2 * modulus: one conditional subtraction
-                uint64_t d[4];
-                unsigned __int128 borrow = 0;
-                for (int j = 0; j < 4; ++j)
-                {
-                    const u128 w = static_cast<u128>(t[j]) - modulus[j] - static_cast<uint64_t>(borrow);
-                    d[j] = static_cast<uint64_t>(w);
-                    borrow = (w >> 64) & 1;
-                }
-                const bool keep = t[4] == 0 && borrow != 0;
-                for (int j = 0; j < 4; ++j) out[j] = keep ? t[j] : d[j];
-            }
-        };
-        // product of two canonical elements, canonical: (a R^2 / R) b / R
-        Fr host_mul_canonical(const Fr& a, const Fr& b)
-        {
-            static const HostFr64 f;
-            uint64_t x[4], y[4], ar[4], out[4];
-            std::memcpy(x, a.l, 32);
-            std::memcpy(y, b.l, 32);
-            f.mul(x, f.r2, ar);
-            f.mul(ar, y, out);
-            Fr r;
-            std::memcpy(r.l, out, 32);
-            return r;
-        }
     }
 
     // Host-side scalar arithmetic for the O(#columns) glue of a caller (same limb code as the

@@ -133,3 +133,61 @@ def test_sumcheck_rounds_fold_to_the_multilinear_evaluation(be):
         assert np.array_equal(cur_host, ora.fold(ora.fr_binop(0, cur.download() if cur.kind == 0 else cur.download(), np.zeros((n, 32), np.uint8)), r))
         cur, n = nxt, half
     assert fr_ints(cur_host)[0] == claim
+
+
+# tiles of 256 and of 1024 elements, odd and even numbers of stages in the first and in later passes, one-stage passes
+@pytest.mark.parametrize("log2n,batch", [(1, 3), (2, 1), (3, 5), (4, 1), (6, 3), (7, 1), (8, 2), (8, 1300), (9, 1), (9, 700), (10, 400), (11, 1), (11, 170), (12, 4),
+                                         (14, 3), (15, 1), (16, 5), (17, 1), (17, 3), (18, 1), (19, 1)])
+def test_ntt_tilings(be, log2n, batch):
+    from project_b200 import KIND_FR, KIND_I64
+
+    rng = np.random.default_rng(1000 * log2n + batch)
+    n = 1 << log2n
+    a = rand_fr(rng, n * batch)
+    buf = be.upload(a, KIND_FR)
+    shift = fr_array([0x1234567 + log2n])
+    checked = sorted({0, batch // 2, batch - 1})
+    for inverse in (False, True):
+        for coset in (None, shift):
+            out = be.ntt(buf, log2n, batch=batch, inverse=inverse, coset_shift=coset).download().reshape(batch, n, 32)
+            for b in checked:
+                assert np.array_equal(out[b], ora.ntt(a.reshape(batch, n, 32)[b], inverse=inverse, coset_shift=coset)), (inverse, b)
+    small = rng.integers(-(1 << 40), 1 << 40, size=n * batch)
+    out = be.ntt(be.upload(small, KIND_I64), log2n, batch=batch).download().reshape(batch, n, 32)
+    want = ora.ntt(ora.fr_from_i64(small[-n:].astype(np.int64)))
+    assert np.array_equal(out[-1], want)
+
+
+@pytest.mark.parametrize("log2n,blowup", [(0, 0), (0, 3), (1, 1), (7, 1), (8, 0), (10, 1), (13, 2), (18, 1)])
+def test_coset_lde_sizes(be, log2n, blowup):
+    from project_b200 import KIND_FR
+
+    rng = np.random.default_rng(log2n)
+    n = 1 << log2n
+    evals = rand_fr(rng, n)
+    shift = fr_array([7 + log2n])
+    padded = np.zeros((n << blowup, 32), dtype=np.uint8)
+    padded[:n] = ora.ntt(evals, inverse=True)
+    got = be.coset_lde(be.upload(evals, KIND_FR), log2n, blowup, shift).download()
+    assert np.array_equal(got, ora.ntt(padded, coset_shift=shift))
+
+
+@pytest.mark.parametrize("n", [2, 3, 64, 511, 514, 300000, 700001])  # one CTA, a few, more rows than the CTAs have threads
+@pytest.mark.parametrize("kind", ["fr", "mont", "i64"])
+def test_sumcheck_round_sums_sizes(be, n, kind):
+    from project_b200 import KIND_FR, KIND_FR_MONT, KIND_I64
+    from pyref import R, fr_ints
+
+    rng = np.random.default_rng(n)
+    if kind == "i64":
+        a = rng.integers(-(1 << 62), 1 << 62, size=n)
+        values = [int(v) for v in a]
+        buf = be.upload(a, KIND_I64)
+    else:
+        a = rand_fr(rng, n)
+        values = fr_ints(a)
+        buf = be.upload(a, KIND_FR if kind == "fr" else KIND_FR_MONT)
+    half = n // 2
+    s0, s1 = sum(values[0:2 * half:2]) % R, sum(values[1:2 * half:2]) % R
+    for _ in range(2):  # the second call finds the arrival counter as the first left it
+        assert fr_ints(be.sumcheck_round_sums(buf, n)) == [s0, s1, (2 * s1 - s0) % R]
