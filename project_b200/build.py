@@ -33,7 +33,7 @@ def _stale(target, deps):
 def build(verbose=False, force=False):
     nvcc = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
     os.makedirs(OBJ_DIR, exist_ok=True)
-    headers = [os.path.join(CSRC, f) for f in os.listdir(CSRC) if f.endswith(".cuh")]
+    headers = [os.path.join(CSRC, f) for f in os.listdir(CSRC) if f.endswith((".cuh", ".hpp"))]
     headers.append(os.path.join(os.path.dirname(HERE), "include", "gatzk_b200.h"))
     headers.append(os.path.join(HERE, "host", "bounded_wait.hpp"))  # included by comm.cu
     jobs = []

@@ -147,11 +147,10 @@ namespace gzk
     // Clears the status word at the start of a call (not in deferred mode, where it is sticky).
     int begin_call(gzk_ctx* ctx);
 
-    // Host-side scalar helpers (same arithmetic, emulated carry flag).
+    // Host-side scalar helpers.
     Fr host_fr_from_bytes(const uint8_t* bytes, bool* canonical_ok);
     void host_fr_to_bytes(const Fr& canonical, uint8_t* bytes);
     Fr host_root_of_unity(unsigned log2n);  // Montgomery form
-    Fr host_fr_mul(const Fr& a, const Fr& b);  // Montgomery product on four 64-bit limbs
 
 #define GZK_CUDA_TRY(ctx, expr)                                         \
     do                                                                  \

@@ -175,98 +175,6 @@ namespace gzk
 
     namespace
     {
-        // Montgomery product on four 64-bit limbs (coarsely integrated operand scanning): the host's
-        // 64x64->128 multiplier does in 32 products what the kernels' 32-bit limb code does in 128.
-        struct HostFr64
-        {
-            uint64_t modulus[4], r2[4], n0;  // n0 = -modulus^-1 mod 2^64
-            HostFr64()
-            {
-                const Fr rr = Fr::r2();
-                for (int i = 0; i < 4; ++i)
-                {
-                    modulus[i] = static_cast<uint64_t>(FrCfg::mod(2 * i)) | (static_cast<uint64_t>(FrCfg::mod(2 * i + 1)) << 32);
-                    r2[i] = static_cast<uint64_t>(rr.l[2 * i]) | (static_cast<uint64_t>(rr.l[2 * i + 1]) << 32);
-                }
-                uint64_t x = 1;  // Newton: x <- x (2 - m x) doubles the correct low bits
-                for (int i = 0; i < 6; ++i) x *= 2 - modulus[0] * x;
-                n0 = ~x + 1;
-            }
-            void mul(const uint64_t a[4], const uint64_t b[4], uint64_t out[4]) const
-            {
-                using u128 = unsigned __int128;
-                uint64_t t[6] = {0, 0, 0, 0, 0, 0};
-                for (int i = 0; i < 4; ++i)
-                {
-                    uint64_t carry = 0;
-                    for (int j = 0; j < 4; ++j)
-                    {
-                        const u128 w = static_cast<u128>(a[j]) * b[i] + t[j] + carry;
-                        t[j] = static_cast<uint64_t>(w);
-                        carry = static_cast<uint64_t>(w >> 64);
-                    }
-                    u128 top = static_cast<u128>(t[4]) + carry;
-                    t[4] = static_cast<uint64_t>(top);
-                    t[5] = static_cast<uint64_t>(top >> 64);
-                    const uint64_t q = t[0] * n0;
-                    u128 w = static_cast<u128>(q) * modulus[0] + t[0];
-                    carry = static_cast<uint64_t>(w >> 64);
-                    for (int j = 1; j < 4; ++j)
-                    {
-                        w = static_cast<u128>(q) * modulus[j] + t[j] + carry;
-                        t[j - 1] = static_cast<uint64_t>(w);
-                        carry = static_cast<uint64_t>(w >> 64);
-                    }
-                    top = static_cast<u128>(t[4]) + carry;
-                    t[3] = static_cast<uint64_t>(top);
-                    t[4] = t[5] + static_cast<uint64_t>(top >> 64);
-                }
-                // t < 2 * modulus: one conditional subtraction
-                uint64_t d[4];
-                unsigned __int128 borrow = 0;
-                for (int j = 0; j < 4; ++j)
-                {
-                    const u128 w = static_cast<u128>(t[j]) - modulus[j] - static_cast<uint64_t>(borrow);
-                    d[j] = static_cast<uint64_t>(w);
-                    borrow = (w >> 64) & 1;
-                }
-                const bool keep = t[4] == 0 && borrow != 0;
-                for (int j = 0; j < 4; ++j) out[j] = keep ? t[j] : d[j];
-            }
-        };
-        const HostFr64& host_fr64()
-        {
-            static const HostFr64 f;
-            return f;
-        }
-        // product of two canonical elements, canonical: (a R^2 / R) b / R
-        Fr host_mul_canonical(const Fr& a, const Fr& b)
-        {
-            const HostFr64& f = host_fr64();
-            uint64_t x[4], y[4], ar[4], out[4];
-            std::memcpy(x, a.l, 32);
-            std::memcpy(y, b.l, 32);
-            f.mul(x, f.r2, ar);
-            f.mul(ar, y, out);
-            Fr r;
-            std::memcpy(r.l, out, 32);
-            return r;
-        }
-    }
-
-    Fr host_fr_mul(const Fr& a, const Fr& b)
-    {
-        uint64_t x[4], y[4], out[4];
-        std::memcpy(x, a.l, 32);
-        std::memcpy(y, b.l, 32);
-        host_fr64().mul(x, y, out);
-        Fr r;
-        std::memcpy(r.l, out, 32);
-        return r;
-    }
-
-    namespace
-    {
         // 5^((r - 1) >> log2n), as FieldElement::root_of_unity divides (r-1) by n
         Fr root_of_unity_by_power(unsigned log2n)
         {
@@ -776,8 +684,7 @@ extern "C"
         return GZK_OK;
     }
 
-    // Host-side scalar arithmetic for the O(#columns) glue of a caller (same limb code as the
-    // kernels, run on the CPU): op 0 add, 1 sub, 2 mul, 3 inverse of a (b ignored).
+    // Host-side scalar arithmetic for the O(#columns) glue of a caller: op 0 add, 1 sub, 2 mul, 3 inverse of a (b ignored).
     int gzk_fr_op(int op, const uint8_t a[32], const uint8_t b[32], uint8_t out[32])
     {
         if (a == nullptr || out == nullptr || (op != 3 && b == nullptr)) return GZK_E_INVALID;
@@ -791,7 +698,7 @@ extern "C"
         {
         case 0: r = add(x, y); break;
         case 1: r = sub(x, y); break;
-        case 2: r = host_mul_canonical(x, y); break;
+        case 2: r = mul(to_mont(x), y); break;
         case 3:
             if (x.is_zero()) return GZK_E_DOMAIN;  // FieldElement::inv throws on zero
             r = from_mont(inv(to_mont(x)));

@@ -10,7 +10,16 @@
 // accumulators (the odd-aligned one becomes even-aligned).
 #pragma once
 
+#include "host_mont.hpp"
 #include "mp.cuh"
+
+// The host pass of the library computes on 64-bit limbs; host programs that compile this header by themselves run
+// the carry chains of the kernels on an emulated carry flag.
+#if defined(__CUDACC__) && !defined(__CUDA_ARCH__)
+#define GZK_HOST_LIMBS 1
+#else
+#define GZK_HOST_LIMBS 0
+#endif
 
 namespace gzk
 {
@@ -135,6 +144,11 @@ namespace gzk
     template <typename Cfg>
     GZK_HD Fe<Cfg> add(const Fe<Cfg>& a, const Fe<Cfg>& b)
     {
+#if GZK_HOST_LIMBS
+        Fe<Cfg> host;
+        HostMont<Cfg>::add(a.l, b.l, host.l);
+        return host;
+#else
         constexpr int N = Cfg::N;
         // Both moduli leave the top bit of the top limb free, so a+b fits N limbs.
         Fe<Cfg> s;
@@ -143,11 +157,17 @@ namespace gzk
         for (int i = 1; i < N - 1; ++i) s.l[i] = mp::addc_cc(a.l[i], b.l[i]);
         s.l[N - 1] = mp::addc(a.l[N - 1], b.l[N - 1]);
         return reduce_once(s);
+#endif
     }
 
     template <typename Cfg>
     GZK_HD Fe<Cfg> sub(const Fe<Cfg>& a, const Fe<Cfg>& b)
     {
+#if GZK_HOST_LIMBS
+        Fe<Cfg> host;
+        HostMont<Cfg>::sub(a.l, b.l, host.l);
+        return host;
+#else
         constexpr int N = Cfg::N;
         Fe<Cfg> d;
         d.l[0] = mp::sub_cc(a.l[0], b.l[0]);
@@ -160,6 +180,7 @@ namespace gzk
         for (int i = 1; i < N - 1; ++i) o.l[i] = mp::addc_cc(d.l[i], borrow & Cfg::mod(i));
         o.l[N - 1] = mp::addc(d.l[N - 1], borrow & Cfg::mod(N - 1));
         return o;
+#endif
     }
 
     template <typename Cfg>
@@ -249,6 +270,11 @@ namespace gzk
     template <typename Cfg>
     GZK_HD Fe<Cfg> mul(const Fe<Cfg>& a, const Fe<Cfg>& b)
     {
+#if GZK_HOST_LIMBS
+        Fe<Cfg> host;
+        HostMont<Cfg>::mul(a.l, b.l, host.l);
+        return host;
+#else
         constexpr int N = Cfg::N;
         static_assert(N % 2 == 0, "limb count must be even");
         uint32_t X[N + 1], Y[N + 1];
@@ -282,6 +308,7 @@ namespace gzk
         for (int k = 1; k < N - 1; ++k) s.l[k] = mp::addc_cc(Y[k + 1], X[k]);
         s.l[N - 1] = mp::addc(Y[N], X[N - 1]);
         return reduce_once(s);
+#endif
     }
 
     template <typename Cfg>

@@ -25,43 +25,85 @@ namespace gzk
 
         // ---- Horner ------------------------------------------------------------------
         // CTA b owns coefficients [b*span, (b+1)*span).  Thread t runs Horner in x^T over
-        // the coefficients s+t, s+t+T, ... (coalesced across the CTA), scales by x^t; the
-        // CTA sum is scaled by x^s.  One Montgomery multiplication per coefficient: the coefficients
+        // the coefficients s+t, s+t+T, ... (coalesced across the CTA); the threads' values join in a tree,
+        // a + x^(2^k) a' at distance 2^k, eight multiplications deep for the CTA (scaling each by x^t first took
+        // sixteen).  The CTA that arrives last (nobody waits) joins the CTA sums the same way with y = x^span.  One
+        // Montgomery multiplication per coefficient: the coefficients
         // enter as stored (x in Montgomery form times a canonical value stays canonical), so a canonical
         // matrix gives the canonical result directly and a Montgomery one is converted at the end.
-        __global__ void __launch_bounds__(kThreads) horner_kernel(ColRef coeffs, uint64_t total, uint64_t span, Fr x, Fr x_stride,
-                                                                  Fr* partial)
+        // Most calls of a proof are one such chain over a few thousand coefficients: PLACEHOLDER
+        struct HornerArgs
         {
-            __shared__ Fr warp_sum[kThreads / 32];
-            const uint64_t s = static_cast<uint64_t>(blockIdx.x) * span;
-            const uint64_t e_end = s + span < total ? s + span : total;
+            ColRef coeffs;
+            uint64_t total, span;
+            Fr x[9], y[9];  // x^(2^k), (x^span)^(2^k): up to x^T
+            int down;       // > 0: that many conversions of the result out of Montgomery form; < 0: into it
+            Fr* partial;    // one per CTA
+            uint32_t* arrived;
+            Fr* out;
+        };
+        // sum over threads t < count of powers[0]^t * value_t, for thread 0; a thread beyond `count` holds zero.
+        // `slots`: one per warp, not in use by anyone when the CTA enters.
+        __device__ __forceinline__ Fr join_powers(Fr value, const Fr* powers, uint32_t count, Fr* slots)
+        {
+            const uint32_t lane = threadIdx.x & 31;
+#pragma unroll 1
+            for (uint32_t k = 0; k < 5 && (1u << k) < count; ++k)
+                value = add(value, mul(powers[k], shfl_fr_idx(value, (lane + (1u << k)) & 31)));
+            if (count <= 32) return value;
+            if (lane == 0) slots[threadIdx.x >> 5] = value;
+            __syncthreads();
+            if (threadIdx.x >= 32) return value;
+            value = lane < kThreads / 32 ? slots[lane] : Fr::zero();
+#pragma unroll 1
+            for (uint32_t k = 5; k < 8 && (1u << k) < count; ++k)
+                value = add(value, mul(powers[k], shfl_fr_idx(value, (lane + (1u << (k - 5))) & 31)));
+            return value;
+        }
+        __global__ void __launch_bounds__(kThreads) horner_kernel(HornerArgs a)
+        {
+            __shared__ Fr slots[kThreads / 32];
+            __shared__ bool last;
+            const uint64_t s = static_cast<uint64_t>(blockIdx.x) * a.span;
+            const uint64_t e_end = s + a.span < a.total ? s + a.span : a.total;
             Fr acc = Fr::zero();
             if (s + threadIdx.x < e_end)
             {
                 const uint64_t steps = (e_end - s - threadIdx.x - 1) / kThreads;  // last index = s + t + steps*T
-                for (uint64_t j = steps + 1; j-- > 0;)
+                acc = col_load_stored(a.coeffs, s + threadIdx.x + steps * kThreads);
+                for (uint64_t j = steps; j-- > 0;)
                 {
-                    acc = mul(acc, x_stride);
-                    acc = add(acc, col_load_stored(coeffs, s + threadIdx.x + j * kThreads));
+                    acc = mul(acc, a.x[8]);
+                    acc = add(acc, col_load_stored(a.coeffs, s + threadIdx.x + j * kThreads));
                 }
-                acc = mul(acc, pow_u64(x, threadIdx.x));
             }
-            const int lane = threadIdx.x & 31;
-#pragma unroll
-            for (int offset = 16; offset > 0; offset >>= 1)
+            const uint64_t owned = e_end - s;
+            acc = join_powers(acc, a.x, owned < kThreads ? static_cast<uint32_t>(owned) : kThreads, slots);
+            if (gridDim.x > 1)
             {
-                const Fr other = shfl_fr_idx(acc, (lane + offset) & 31);
-                if (lane < offset) acc = add(acc, other);
+                if (threadIdx.x == 0)
+                {
+                    store_fr(a.partial + blockIdx.x, acc);
+                    __threadfence();
+                    last = atomicAdd(a.arrived, 1u) + 1 == gridDim.x;
+                }
+                __syncthreads();
+                if (!last) return;
+                __threadfence();
+                acc = Fr::zero();
+                for (uint32_t j = (gridDim.x - 1) / kThreads + 1; j-- > 0;)
+                {
+                    const uint32_t b = j * kThreads + threadIdx.x;
+                    acc = mul(acc, a.y[8]);
+                    if (b < gridDim.x) acc = add(acc, load_fr_plain(a.partial + b));
+                }
+                acc = join_powers(acc, a.y, gridDim.x < kThreads ? gridDim.x : kThreads, slots);
+                if (threadIdx.x == 0) *a.arrived = 0;  // for the next call
             }
-            if (lane == 0) warp_sum[threadIdx.x >> 5] = acc;
-            __syncthreads();
-            if (threadIdx.x == 0)
-            {
-                Fr sum = warp_sum[0];
-#pragma unroll
-                for (int w = 1; w < kThreads / 32; ++w) sum = add(sum, warp_sum[w]);
-                store_fr(partial + blockIdx.x, mul(sum, pow_u64(x, s)));
-            }
+            if (threadIdx.x != 0) return;
+            for (int d = a.down; d > 0; --d) acc = from_mont(acc);
+            for (int d = a.down; d < 0; ++d) acc = to_mont(acc);
+            store_fr(a.out, acc);
         }
 
         // Matrix entries by buffer kind, resolved at compile time so that a kernel can issue the loads of
@@ -233,17 +275,6 @@ namespace gzk
                     store_fr(out + b, value);
                 }
             }
-        }
-
-        // `down` > 0: that many conversions out of Montgomery form; < 0: into it.
-        __global__ void sum_partials_kernel(const Fr* partial, uint32_t count, int down, Fr* out)
-        {
-            if (threadIdx.x != 0 || blockIdx.x != 0) return;
-            Fr sum = Fr::zero();
-            for (uint32_t i = 0; i < count; ++i) sum = add(sum, load_fr_plain(partial + i));
-            for (; down > 0; --down) sum = from_mont(sum);
-            for (; down < 0; ++down) sum = to_mont(sum);
-            store_fr(out, sum);
         }
 
         // ---- fold rows ----------------------------------------------------------------
@@ -474,10 +505,44 @@ namespace gzk
             store_fr(out + row, value);
         }
 
-        __global__ void powers_kernel(Fr c, uint64_t count, Fr* out)
+        // out[i] = c^i as the product of the c^(2^k) of i's bits: half as many multiplications as bits (squaring on the
+        // way, per thread, took up to twice as many as bits: 1024 powers 17 us, now PLACEHOLDER2).  `bias_out`,
+        // where given, receives `bias` (the constant that belongs to these powers).
+        struct PowersArgs
+        {
+            Fr square[40];  // c^(2^k)
+            uint64_t count;
+            Fr* out;
+            Fr bias;
+            Fr* bias_out;
+        };
+        __global__ void powers_kernel(PowersArgs a)
         {
             const uint64_t i = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-            if (i < count) store_fr(out + i, pow_u64(c, i));
+            if (i >= a.count) return;
+            if (i == 0 && a.bias_out != nullptr) store_fr(a.bias_out, a.bias);
+            Fr v = Fr::one();
+            bool started = false;
+#pragma unroll 1
+            for (uint32_t k = 0; (i >> k) != 0; ++k)
+            {
+                if (((i >> k) & 1u) == 0) continue;
+                v = started ? mul(v, a.square[k]) : a.square[k];
+                started = true;
+            }
+            store_fr(a.out + i, v);
+        }
+        void launch_powers(gzk_ctx* ctx, const Fr& c, uint64_t count, Fr* out, const Fr* bias, Fr* bias_out)
+        {
+            PowersArgs args;
+            args.square[0] = c;
+            for (int k = 1; k < 40; ++k) args.square[k] = (count >> k) != 0 ? sqr(args.square[k - 1]) : Fr::zero();
+            args.count = count;
+            args.out = out;
+            args.bias = bias != nullptr ? *bias : Fr::zero();
+            args.bias_out = bias != nullptr ? bias_out : nullptr;
+            LaunchScope scope(ctx, "powers");
+            powers_kernel<<<static_cast<unsigned>((count + 127) / 128), 128, 0, ctx->stream>>>(args);
         }
 
         // 2^31 in Montgomery form
@@ -517,7 +582,8 @@ extern "C"
         const bool blocked = small_kind && total >= (1u << 16);
         const uint64_t dot_blocks = blocked ? (total + kDotBlock - 1) / kDotBlock : 0;
         const uint64_t horner_total = blocked ? dot_blocks : total;
-        uint64_t ctas = (horner_total + static_cast<uint64_t>(kThreads) * 8 - 1) / (static_cast<uint64_t>(kThreads) * 8);
+        // four coefficients per thread: a chain of three multiplications before the trees
+        uint64_t ctas = (horner_total + static_cast<uint64_t>(kThreads) * 4 - 1) / (static_cast<uint64_t>(kThreads) * 4);
         const uint64_t max_ctas = static_cast<uint64_t>(ctx->sm_count) * 8;
         if (ctas > max_ctas) ctas = max_ctas;
         uint64_t span = (horner_total + ctas - 1) / ctas;
@@ -539,14 +605,16 @@ extern "C"
             Fr* powers = partial + ctas + 1;
             Fr* bias = powers + kDotBlock;
             Fr* block_values = bias + 1;
+            // many blocks of I64 coefficients: the block sums are a row-wise linear form of a dot_blocks x 1024 matrix
+            // and run on the tensor cores (entries biased by 2^63 there, by 2^31 in block_dot_kernel); the bias times
+            // the sum of the powers is sum_(j < 1024) x^j = prod_k (1 + x^(2^k)) times it
+            Fr bias_value = tensor_blocks ? mont_two_63() : mont_two_31(), square = x;
+            for (int width = 1; width < kDotBlock; width *= 2)
             {
-                LaunchScope scope(ctx, "powers");
-                powers_kernel<<<kDotBlock / kThreads, kThreads, 0, ctx->stream>>>(x, kDotBlock, powers);
-                // many blocks of I64 coefficients: the block sums are a row-wise linear form of a dot_blocks x 1024 matrix
-                // and run on the tensor cores (entries biased by 2^63 there, by 2^31 in block_dot_kernel)
-                if (matrix->kind == GZK_KIND_I64)
-                    scaled_sum_kernel<<<1, kThreads, 0, ctx->stream>>>(powers, kDotBlock, tensor_blocks ? mont_two_63() : mont_two_31(), bias);
+                bias_value = mul(bias_value, add(Fr::one(), square));
+                square = sqr(square);
             }
+            launch_powers(ctx, x, kDotBlock, powers, &bias_value, bias);
             GZK_CUDA_TRY(ctx, cudaGetLastError());
             const uint64_t warps_wanted = dot_blocks < static_cast<uint64_t>(ctx->sm_count) * 64 ? dot_blocks : static_cast<uint64_t>(ctx->sm_count) * 64;
             {
@@ -564,18 +632,27 @@ extern "C"
             m.kind = GZK_KIND_FR_MONT;
             x_horner = pow_u64(x, kDotBlock);
         }
+        Fr* result = dest != nullptr ? dest : partial + ctas;
+        HornerArgs args;
+        args.coeffs = m;
+        args.total = horner_total;
+        args.span = span;
+        args.x[0] = x_horner;
+        args.y[0] = pow_u64(x_horner, span);
+        for (int k = 1; k <= 8; ++k)
+        {
+            args.x[k] = sqr(args.x[k - 1]);
+            args.y[k] = sqr(args.y[k - 1]);
+        }
+        // the sum is the Montgomery form of the canonical result (canonical entries) or of its Montgomery form
+        // (Montgomery entries): one or two conversions bring it to the wanted form
+        args.down = (m.kind == GZK_KIND_FR_MONT ? 1 : 0) - (dest_montgomery ? 1 : 0);
+        args.partial = partial;
+        args.arrived = ctx->arrival_counter();
+        args.out = result;
         {
             LaunchScope scope(ctx, "horner");
-            horner_kernel<<<static_cast<unsigned>(ctas), kThreads, 0, ctx->stream>>>(m, horner_total, span, x_horner, pow_u64(x_horner, kThreads), partial);
-        }
-        GZK_CUDA_TRY(ctx, cudaGetLastError());
-        Fr* result = dest != nullptr ? dest : partial + ctas;
-        {
-            // the partial sums are Montgomery values of the canonical result (canonical entries) or of its
-            // Montgomery form (Montgomery entries): one or two conversions bring them to the wanted form
-            LaunchScope scope(ctx, "horner_sum");
-            const int down = (m.kind == GZK_KIND_FR_MONT ? 1 : 0) - (dest_montgomery ? 1 : 0);
-            sum_partials_kernel<<<1, 32, 0, ctx->stream>>>(partial, static_cast<uint32_t>(ctas), down, result);
+            horner_kernel<<<static_cast<unsigned>(ctas), kThreads, 0, ctx->stream>>>(args);
         }
         GZK_CUDA_TRY(ctx, cudaGetLastError());
         if (scratch_result != nullptr) *scratch_result = result;
@@ -787,10 +864,7 @@ extern "C"
         int rc = scalar_mont(ctx, challenge, &c);
         if (rc != GZK_OK) return rc;
         GZK_CUDA_TRY(ctx, cudaSetDevice(ctx->device));
-        {
-            LaunchScope scope(ctx, "powers");
-            powers_kernel<<<static_cast<unsigned>((count + 127) / 128), 128, 0, ctx->stream>>>(c, count, static_cast<Fr*>(out->dptr));
-        }
+        launch_powers(ctx, c, count, static_cast<Fr*>(out->dptr), nullptr, nullptr);
         GZK_CUDA_TRY(ctx, cudaGetLastError());
         return finish_call(ctx, "invalid input");
     }

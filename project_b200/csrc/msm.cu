@@ -36,11 +36,11 @@ namespace gzk
     {
         constexpr int kThreads = 128;
         constexpr int kMaxWindows = 32;
-        // Buckets with more entries than kBigBucket (skewed scalars: small integers, constant
+        // Buckets with more than four times the mean of their plan (`big`; skewed scalars: small integers, constant
         // columns, the short top window) are cut into slices; one CTA sums a slice, one CTA then adds the
         // slices of a bucket.  Short slices make the chains short (a thread adds four points of a slice of
         // 512, and a quad of lanes joins them), and a very long bucket has at most 256.
-        constexpr uint32_t kBigBucket = 1024;
+        constexpr uint32_t kBigBucketMin = 128, kBigBucketMax = 1024;
         constexpr uint32_t kSliceEntries = 512;
         constexpr uint32_t kMaxSlices = 256;
         __device__ __forceinline__ uint32_t slice_entries(uint32_t size)
@@ -163,21 +163,21 @@ namespace gzk
         // by their square root, so that the longest of 32 holds a fifth more than the mean at 240 points and two
         // thirds more at 16), and the last warps to start have the least to do.  Buckets the slices take come last,
         // with size 0.
-        constexpr uint32_t kSizeBins = kBigBucket + 1;
-        __device__ __forceinline__ uint32_t size_bin(uint32_t size) { return size > kBigBucket ? kBigBucket : kBigBucket - size; }
-        __global__ void __launch_bounds__(1024) msm_size_histogram_kernel(const uint32_t* bucket_size, uint32_t buckets, uint32_t* histogram)
+        constexpr uint32_t kSizeBins = kBigBucketMax + 1;
+        __device__ __forceinline__ uint32_t size_bin(uint32_t size, uint32_t big) { return size > big ? kBigBucketMax : kBigBucketMax - size; }
+        __global__ void __launch_bounds__(1024) msm_size_histogram_kernel(const uint32_t* bucket_size, uint32_t buckets, uint32_t big, uint32_t* histogram)
         {
             __shared__ uint32_t local[kSizeBins];
             for (uint32_t i = threadIdx.x; i < kSizeBins; i += blockDim.x) local[i] = 0;
             __syncthreads();
             const uint32_t b = blockIdx.x * blockDim.x + threadIdx.x;
-            if (b < buckets) atomicAdd(local + size_bin(bucket_size[b]), 1u);
+            if (b < buckets) atomicAdd(local + size_bin(bucket_size[b], big), 1u);
             __syncthreads();
             for (uint32_t i = threadIdx.x; i < kSizeBins; i += blockDim.x)
                 if (local[i] != 0) atomicAdd(histogram + i, local[i]);
         }
         // `cursor`: one zeroed word per bin
-        __global__ void __launch_bounds__(1024) msm_order_kernel(const uint32_t* bucket_size, uint32_t buckets, const uint32_t* histogram, uint32_t* cursor, uint32_t* order)
+        __global__ void __launch_bounds__(1024) msm_order_kernel(const uint32_t* bucket_size, uint32_t buckets, uint32_t big, const uint32_t* histogram, uint32_t* cursor, uint32_t* order)
         {
             __shared__ uint32_t first[kSizeBins], local[kSizeBins];
             __shared__ uint32_t warp_totals[32];
@@ -204,7 +204,7 @@ namespace gzk
             uint32_t bin = 0, rank = 0;
             if (b < buckets)
             {
-                bin = size_bin(bucket_size[b]);
+                bin = size_bin(bucket_size[b], big);
                 rank = atomicAdd(local + bin, 1u);
             }
             __syncthreads();
@@ -251,13 +251,13 @@ namespace gzk
         template <int LANES>
         __global__ void __launch_bounds__(kThreads) msm_buckets_kernel(const G1Affine* points, const uint32_t* bucket_start,
                                                                       const uint32_t* bucket_size, const uint32_t* order, const uint32_t* entries,
-                                                                      uint32_t buckets, G1Xyzz* out)
+                                                                      uint32_t buckets, uint32_t big, G1Xyzz* out)
         {
             const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
             const uint32_t slot = t / LANES, part = t % LANES;
             const uint32_t b = slot < buckets ? order[slot] : 0;
             const uint32_t start = bucket_start[b], size = slot < buckets ? bucket_size[b] : 0;
-            const bool mine = size <= kBigBucket;  // longer ones are handled cooperatively by msm_big_slices_kernel
+            const bool mine = size <= big;  // longer ones are handled cooperatively by msm_big_slices_kernel
             G1Xyzz acc = G1Xyzz::infinity();
             if (mine)
             {
@@ -278,13 +278,13 @@ namespace gzk
         }
 
         // counters[0] = number of slice items, counters[1] = number of big buckets
-        __global__ void __launch_bounds__(kThreads) msm_plan_big_kernel(const uint32_t* bucket_size, uint32_t buckets, uint32_t* counters,
+        __global__ void __launch_bounds__(kThreads) msm_plan_big_kernel(const uint32_t* bucket_size, uint32_t buckets, uint32_t threshold, uint32_t* counters,
                                                                        BigItem* items, BigBucket* big)
         {
             const uint32_t b = blockIdx.x * blockDim.x + threadIdx.x;
             if (b >= buckets) return;
             const uint32_t size = bucket_size[b];
-            if (size <= kBigBucket) return;
+            if (size <= threshold) return;
             const uint32_t entries = slice_entries(size), slices = (size + entries - 1) / entries;
             const uint32_t first = atomicAdd(counters, slices);
             const uint32_t slot = atomicAdd(counters + 1, 1u);
@@ -515,7 +515,7 @@ namespace gzk
             {
                 const int windows = (256 + c - 1) / c, top_bits = 255 - c * (windows - 1);
                 double cost = 10.0 * static_cast<double>(n) * windows + 45.0 * windows * static_cast<double>(1u << (c - 1));
-                if (static_cast<double>(n) > static_cast<double>(kBigBucket) * static_cast<double>(1u << top_bits)) cost += 5.0 * static_cast<double>(n);
+                if (top_bits < c - 3) cost += 5.0 * static_cast<double>(n);
                 if (best_cost == 0.0 || cost < best_cost)
                 {
                     best_cost = cost;
@@ -525,14 +525,16 @@ namespace gzk
             return best;
         }
 
-        // Lanes per bucket: as many as leave eight warps for every scheduler and two points for every lane.  One lane
-        // per bucket left 13312 lanes for 2^16 points: bucket pass 1773 us, with window and lanes chosen as here 662 us
-        // (whole call 5.27 -> 1.37 ms); 2^20 points on their table, 240 to a bucket: 7.93 -> 6.89 ms (call 9.36 -> 7.75 ms).
+        // Lanes per bucket: two points for every lane until each scheduler has four warps, sixteen until it has
+        // sixteen (more warps even out the last wave; joining the lanes costs as much as 1.4 points a level).  One
+        // lane per bucket left 13312 lanes for 2^16 points: bucket pass 1773 us, with window and lanes chosen as here
+        // 662 us (whole call 5.27 -> 1.37 ms).  2^20 points on their table, 240 to a bucket: call 8.43 / 7.74 / 7.44 ms
+        // with 1 / 2 / 4 lanes (9.36 ms before the buckets were ordered).
         uint32_t bucket_lanes(const gzk_ctx* ctx, uint64_t buckets, uint64_t entries)
         {
-            const uint64_t threads = static_cast<uint64_t>(ctx->sm_count) * 4 * 8 * 32;
+            const uint64_t four_warps = static_cast<uint64_t>(ctx->sm_count) * 4 * 4 * 32;
             uint32_t lanes = 1;
-            while (lanes < 8 && buckets * lanes * 2 <= threads && entries >= buckets * lanes * 4) lanes *= 2;
+            while (lanes < 8 && buckets * lanes * 2 <= (entries >= buckets * lanes * 32 ? 4 * four_warps : four_warps) && entries >= buckets * lanes * 4) lanes *= 2;
 #ifdef GZK_BUILD_TUNING
             if (const char* forced = std::getenv("GZK_MSM_LANES")) lanes = static_cast<uint32_t>(std::atoi(forced));
 #endif
@@ -561,7 +563,9 @@ namespace gzk
         const size_t code_bytes = static_cast<size_t>(n) * plan.windows * sizeof(uint32_t);
         const size_t bucket_u32 = buckets * sizeof(uint32_t);
         const uint64_t total_entries = n * plan.windows;
-        const uint64_t max_big = total_entries / kBigBucket + 1;          // buckets that can exceed the threshold
+        const uint64_t four_means = 4 * total_entries / buckets;
+        const uint32_t big = four_means < kBigBucketMin ? kBigBucketMin : four_means > kBigBucketMax ? kBigBucketMax : static_cast<uint32_t>(four_means);
+        const uint64_t max_big = total_entries / big + 1;          // buckets that can exceed the threshold
         const uint64_t max_items = total_entries / kSliceEntries + max_big; // sum of ceil(size / slice) over them
         const size_t big_bytes = max_items * (sizeof(BigItem) + sizeof(G1Xyzz)) + max_big * sizeof(BigBucket) + 64;
         const uint32_t split_h = (plan.c - 1) / 2;                          // low bits of the bucket multiplier
@@ -624,15 +628,15 @@ namespace gzk
         {
             LaunchScope scope(ctx, "msm_plan_big");
             msm_plan_big_kernel<<<static_cast<unsigned>((buckets + kThreads - 1) / kThreads), kThreads, 0, ctx->stream>>>(
-                bucket_size, static_cast<uint32_t>(buckets), big_counters, big_items, big_buckets);
+                bucket_size, static_cast<uint32_t>(buckets), big, big_counters, big_items, big_buckets);
         }
         GZK_CUDA_TRY(ctx, cudaGetLastError());
         GZK_CUDA_TRY(ctx, cudaMemsetAsync(size_bins, 0, 2 * kSizeBins * sizeof(uint32_t), ctx->stream));
         {
             LaunchScope scope(ctx, "msm_order", 2);
             const unsigned blocks = static_cast<unsigned>((buckets + 1023) / 1024);
-            msm_size_histogram_kernel<<<blocks, 1024, 0, ctx->stream>>>(bucket_size, static_cast<uint32_t>(buckets), size_bins);
-            msm_order_kernel<<<blocks, 1024, 0, ctx->stream>>>(bucket_size, static_cast<uint32_t>(buckets), size_bins, size_bins + kSizeBins, order);
+            msm_size_histogram_kernel<<<blocks, 1024, 0, ctx->stream>>>(bucket_size, static_cast<uint32_t>(buckets), big, size_bins);
+            msm_order_kernel<<<blocks, 1024, 0, ctx->stream>>>(bucket_size, static_cast<uint32_t>(buckets), big, size_bins, size_bins + kSizeBins, order);
         }
         GZK_CUDA_TRY(ctx, cudaGetLastError());
         {
@@ -640,7 +644,7 @@ namespace gzk
             const uint32_t lanes = bucket_lanes(ctx, buckets, total_entries);
             const auto kernel = lanes == 1 ? msm_buckets_kernel<1> : lanes == 2 ? msm_buckets_kernel<2> : lanes == 4 ? msm_buckets_kernel<4> : msm_buckets_kernel<8>;
             kernel<<<static_cast<unsigned>((buckets * lanes + kThreads - 1) / kThreads), kThreads, 0, ctx->stream>>>(
-                static_cast<const G1Affine*>(points->dptr), bucket_start, bucket_size, order, entries, static_cast<uint32_t>(buckets), bucket_points);
+                static_cast<const G1Affine*>(points->dptr), bucket_start, bucket_size, order, entries, static_cast<uint32_t>(buckets), big, bucket_points);
         }
         GZK_CUDA_TRY(ctx, cudaGetLastError());
         {
@@ -667,8 +671,8 @@ namespace gzk
         }
         GZK_CUDA_TRY(ctx, cudaGetLastError());
         // the shifts of the windows are one chain of c * w doublings: the host's part
-        HostXyzz sums[kMaxWindows];
-        GZK_CUDA_TRY(ctx, cudaMemcpyAsync(sums, window_sums, bucket_sets * sizeof(HostXyzz), cudaMemcpyDeviceToHost, ctx->stream));
+        G1Xyzz sums[kMaxWindows];
+        GZK_CUDA_TRY(ctx, cudaMemcpyAsync(sums, window_sums, bucket_sets * sizeof(G1Xyzz), cudaMemcpyDeviceToHost, ctx->stream));
         GZK_CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream));
         host_to_affine_bytes(host_horner(sums, bucket_sets, plan.c), out_host);
         return GZK_OK;

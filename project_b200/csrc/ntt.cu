@@ -445,7 +445,7 @@ static int ntt_run(gzk_ctx* ctx, const ColRef& in, uint64_t in_count, Fr* out, u
         powers.lo = static_cast<Fr*>(scratch);
         powers.hi = powers.lo + lo_count;
         powers.square[0] = pre != nullptr ? *pre : *post;
-        for (unsigned k = 1; k < log2n; ++k) powers.square[k] = host_fr_mul(powers.square[k - 1], powers.square[k - 1]);
+        for (unsigned k = 1; k < log2n; ++k) powers.square[k] = sqr(powers.square[k - 1]);
         powers.factor = post != nullptr && inverse ? args.scale : Fr::one();
         {
             LaunchScope scope(ctx, "ntt_shift_table");
