@@ -127,6 +127,9 @@ int gzk_host_unregister(void* host);
 /* downloads always deliver the wire format: FR_MONT buffers are converted to
  * canonical on the device first */
 int gzk_buf_download(gzk_ctx* ctx, const gzk_buf* buf, size_t offset, void* host, size_t count);
+/* out[i] = element indices[i] of bufs[i] (FR or FR_MONT buffers), 32 canonical bytes each: single values of many
+ * columns with one wait */
+int gzk_buf_download_elements(gzk_ctx* ctx, const gzk_buf* const* bufs, const uint64_t* indices, size_t count, uint8_t* out);
 size_t gzk_buf_count(const gzk_buf* buf);
 int gzk_buf_kind(const gzk_buf* buf);
 void* gzk_buf_device_ptr(gzk_buf* buf);

@@ -3,7 +3,16 @@
 // multiplication [p_k(tau)] G per column; and the honest-prover alternative, a
 // Lagrange-basis SRS [L_i(tau)] G against which a column is committed by an MSM
 // (same group element, because sum_i f_i [L_i(tau)] G = [sum_i f_i L_i(tau)] G).
+#include <cstring>
+
 #include "common.cuh"
+
+namespace gzk
+{
+    int eval_batch_enqueue(gzk_ctx* ctx, gzk_buf* const* cols, size_t k_count, size_t len, unsigned log2n, const gzk_buf* weights, Fr* dest);
+    int eval_status_error(gzk_ctx* ctx, int status);
+    int g1_same_base_enqueue(gzk_ctx* ctx, const uint8_t base[96], const Fr* scalars, int kind, size_t count, uint8_t* out_pinned);
+}
 
 using namespace gzk;
 
@@ -15,10 +24,22 @@ extern "C"
         if (ctx == nullptr) return GZK_E_INVALID;
         if (k_count == 0) return GZK_OK;
         if (tau_evals_out == nullptr || points_out == nullptr || base == nullptr) return fail(ctx, GZK_E_INVALID, "commit_batch: null argument");
-        const uint64_t zero_rotation = 0;
-        int rc = gzk_eval_batch(ctx, cols, k_count, len, log2n, weights_tau, &zero_rotation, 1, tau_evals_out);
+        // one wait for both steps: the evaluations stay on the device between them
+        void* d_evals = nullptr;
+        void* h_out = nullptr;
+        int rc = ensure_scratch(ctx, 3, k_count * sizeof(Fr), &d_evals);
         if (rc != GZK_OK) return rc;
-        return gzk_g1_mul_same_base(ctx, base, tau_evals_out, k_count, points_out);
+        if ((rc = eval_batch_enqueue(ctx, cols, k_count, len, log2n, weights_tau, static_cast<Fr*>(d_evals))) != GZK_OK) return rc;
+        if ((rc = ensure_pinned(ctx, k_count * (96 + sizeof(Fr)) + 64, &h_out)) != GZK_OK) return rc;
+        if ((rc = g1_same_base_enqueue(ctx, base, static_cast<const Fr*>(d_evals), GZK_KIND_FR, k_count, static_cast<uint8_t*>(h_out))) != GZK_OK) return rc;
+        uint8_t* h_evals = static_cast<uint8_t*>(h_out) + k_count * 96;
+        GZK_CUDA_TRY(ctx, cudaMemcpyAsync(h_evals, d_evals, k_count * sizeof(Fr), cudaMemcpyDeviceToHost, ctx->stream));
+        GZK_CUDA_TRY(ctx, cudaMemcpyAsync(ctx->h_status, ctx->d_status, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
+        GZK_CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream));
+        if ((rc = eval_status_error(ctx, *ctx->h_status)) != GZK_OK) return rc;
+        std::memcpy(points_out, h_out, k_count * 96);
+        std::memcpy(tau_evals_out, h_evals, k_count * sizeof(Fr));
+        return GZK_OK;
     }
 
     int gzk_srs_lagrange(gzk_ctx* ctx, unsigned log2n, const uint8_t base[96], const uint8_t tau[32], gzk_buf* out_points)

@@ -280,6 +280,24 @@ namespace gzk
         return GZK_OK;
     }
 
+    // out[i] = *src[i], canonical: single values of many columns in one launch
+    constexpr uint32_t kGatherElements = 128;
+    constexpr size_t kSmallDownload = 64u << 10;
+    struct GatherElements
+    {
+        const Fr* src[kGatherElements];
+        uint8_t montgomery[kGatherElements];
+        uint32_t count;
+        Fr* out;
+    };
+    __global__ void gather_elements_kernel(const __grid_constant__ GatherElements a)
+    {
+        const uint32_t i = threadIdx.x;
+        if (i >= a.count) return;
+        const Fr v = load_fr_plain(a.src[i]);
+        store_fr(a.out + i, a.montgomery[i] ? from_mont(v) : v);
+    }
+
     __global__ void convert_kernel(const Fr* in, Fr* out, size_t count, int to_montgomery)
     {
         const size_t stride = static_cast<size_t>(gridDim.x) * blockDim.x;
@@ -628,6 +646,31 @@ extern "C"
         if (offset + count > buf->count) return fail(ctx, GZK_E_INVALID, "download exceeds the buffer");
         if (count == 0) return GZK_OK;
         const char* src = static_cast<const char*>(buf->dptr) + offset * buf->elem_bytes;
+        // A few values, the usual read-back of a proof (evaluations, points, totals): through pinned memory, which the
+        // conversion kernels write directly.
+        if (count * buf->elem_bytes <= kSmallDownload)
+        {
+            void* staging = nullptr;
+            int rc = ensure_pinned(ctx, kSmallDownload, &staging);
+            if (rc != GZK_OK) return rc;
+            if (buf->kind == GZK_KIND_FR_MONT)
+            {
+                LaunchScope scope(ctx, "convert");
+                convert_kernel<<<static_cast<unsigned>((count + 255) / 256), 256, 0, ctx->stream>>>(reinterpret_cast<const Fr*>(src), static_cast<Fr*>(staging), count, 0);
+                GZK_CUDA_TRY(ctx, cudaGetLastError());
+            }
+            else if (buf->kind == GZK_KIND_G1)
+            {
+                if ((rc = launch_convert_fp(ctx, src, staging, count * 2, false)) != GZK_OK) return rc;
+            }
+            else
+            {
+                GZK_CUDA_TRY(ctx, cudaMemcpyAsync(staging, src, count * buf->elem_bytes, cudaMemcpyDeviceToHost, ctx->stream));
+            }
+            GZK_CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream));
+            std::memcpy(host, staging, count * buf->elem_bytes);
+            return GZK_OK;
+        }
         if (buf->kind == GZK_KIND_FR_MONT)
         {
             // convert in chunks through context scratch so that the buffer itself stays Montgomery
@@ -666,6 +709,40 @@ extern "C"
         }
         GZK_CUDA_TRY(ctx, cudaMemcpyAsync(host, src, count * buf->elem_bytes, cudaMemcpyDeviceToHost, ctx->stream));
         GZK_CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream));
+        return GZK_OK;
+    }
+
+    int gzk_buf_download_elements(gzk_ctx* ctx, const gzk_buf* const* bufs, const uint64_t* indices, size_t count, uint8_t* out)
+    {
+        if (ctx == nullptr) return GZK_E_INVALID;
+        if (count == 0) return GZK_OK;
+        if (bufs == nullptr || indices == nullptr || out == nullptr) return fail(ctx, GZK_E_INVALID, "download_elements: null argument");
+        for (size_t i = 0; i < count; ++i)
+        {
+            if (bufs[i] == nullptr || (bufs[i]->kind != GZK_KIND_FR && bufs[i]->kind != GZK_KIND_FR_MONT))
+                return fail(ctx, GZK_E_INVALID, "download_elements: the buffers must hold field elements");
+            if (indices[i] >= bufs[i]->count) return fail(ctx, GZK_E_INVALID, "download exceeds the buffer");
+        }
+        GZK_CUDA_TRY(ctx, cudaSetDevice(ctx->device));
+        void* staging = nullptr;
+        int rc = ensure_pinned(ctx, count * sizeof(Fr), &staging);
+        if (rc != GZK_OK) return rc;
+        for (size_t done = 0; done < count; done += kGatherElements)
+        {
+            GatherElements args{};
+            args.count = static_cast<uint32_t>(count - done < kGatherElements ? count - done : kGatherElements);
+            args.out = static_cast<Fr*>(staging) + done;
+            for (uint32_t i = 0; i < args.count; ++i)
+            {
+                args.src[i] = static_cast<const Fr*>(bufs[done + i]->dptr) + indices[done + i];
+                args.montgomery[i] = bufs[done + i]->kind == GZK_KIND_FR_MONT ? 1 : 0;
+            }
+            LaunchScope scope(ctx, "convert");
+            gather_elements_kernel<<<1, kGatherElements, 0, ctx->stream>>>(args);
+            GZK_CUDA_TRY(ctx, cudaGetLastError());
+        }
+        GZK_CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream));
+        std::memcpy(out, staging, count * sizeof(Fr));
         return GZK_OK;
     }
 

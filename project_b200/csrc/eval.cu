@@ -34,6 +34,7 @@ namespace gzk
         constexpr int kAccLimbs = 17;
         constexpr int kThreads = 128;
 
+        constexpr uint32_t kInlineColumns = 64;
         struct EvalArgs
         {
             const void* const* cols;  // K device pointers
@@ -51,6 +52,15 @@ namespace gzk
             uint32_t skip_copies;     // stall injection (gzk_debug_inject_eval_stall): announce the chunks but issue no copy
             const uint32_t* k_map;    // the columns this launch takes (indices into cols), or null: all k_count of them
             uint32_t k_mapped;        // entries of k_map (k_count without a map)
+            // A call of few columns carries its column table in the launch itself (cols, kinds, k_map null): a copy per call
+            // is one more operation on the stream and on the host, and a proof makes hundreds of such calls.
+            const void* inline_cols[kInlineColumns];
+            uint8_t inline_kinds[kInlineColumns];
+            uint8_t inline_map[kInlineColumns];  // the field-element columns first
+            uint32_t inline_first;               // the launch's columns start here in inline_map
+            __device__ __forceinline__ const void* column(uint32_t k) const { return cols != nullptr ? cols[k] : inline_cols[k]; }
+            __device__ __forceinline__ int kind(uint32_t k) const { return cols != nullptr ? kinds[k] : static_cast<int>(inline_kinds[k]); }
+            __device__ __forceinline__ uint32_t mapped(uint32_t i) const { return cols == nullptr ? inline_map[inline_first + i] : k_map != nullptr ? k_map[i] : i; }
         };
         // Which columns a launch takes.  Field-element columns run through the shared-memory ring and the tensor
         // cores; small-integer columns in groups of four through a tensor-core kernel of their own
@@ -220,7 +230,7 @@ namespace gzk
         }
 
         template <int P, int MODE>
-        __global__ void __launch_bounds__(kThreads, MODE == kIntegerKinds ? (P == 2 ? 4 : 5) : (P == 2 ? 4 : 3)) eval_partial_kernel(EvalArgs a)
+        __global__ void __launch_bounds__(kThreads, MODE == kIntegerKinds ? (P == 2 ? 4 : 5) : (P == 2 ? 4 : 3)) eval_partial_kernel(const __grid_constant__ EvalArgs a)
         {
             constexpr bool kHasField = MODE != kIntegerKinds;
             extern __shared__ __align__(128) unsigned char smem[];
@@ -252,9 +262,9 @@ namespace gzk
             {
                 const uint32_t tile = static_cast<uint32_t>(u / a.k_mapped);
                 const uint32_t slot_of_k = static_cast<uint32_t>(u - static_cast<uint64_t>(tile) * a.k_mapped);
-                const uint32_t k = a.k_map != nullptr ? a.k_map[slot_of_k] : slot_of_k;
-                const void* col = a.cols[k];
-                const int kind = a.kinds[k];
+                const uint32_t k = a.mapped(slot_of_k);
+                const void* col = a.column(k);
+                const int kind = a.kind(k);
                 const uint64_t c_begin = static_cast<uint64_t>(tile) * a.tile_rows;
                 const uint64_t c_end = c_begin + a.tile_rows < a.len ? c_begin + a.tile_rows : a.len;
 
@@ -611,7 +621,7 @@ namespace gzk
         }
 
         template <int P>
-        __global__ void __launch_bounds__(kThreads, 3) eval_integers_kernel(EvalArgs a)
+        __global__ void __launch_bounds__(kThreads, 3) eval_integers_kernel(const __grid_constant__ EvalArgs a)
         {
             extern __shared__ __align__(128) unsigned char smem[];
             __shared__ IntegerScratch scratch_of[kWarps];
@@ -644,9 +654,9 @@ namespace gzk
                 {
                     const uint32_t slot = group * kGroupColumns + c;
                     const bool there = slot < a.k_mapped;
-                    const uint32_t k = there ? a.k_map[slot] : 0;
-                    column_of[c] = there ? static_cast<const unsigned char*>(a.cols[k]) : nullptr;
-                    wide_of[c] = there && a.kinds[k] == GZK_KIND_I64;
+                    const uint32_t k = there ? a.mapped(slot) : 0;
+                    column_of[c] = there ? static_cast<const unsigned char*>(a.column(k)) : nullptr;
+                    wide_of[c] = there && a.kind(k) == GZK_KIND_I64;
                 }
                 const bool present = group * kGroupColumns + my_column < a.k_mapped;
                 bool wide = false;
@@ -763,7 +773,7 @@ namespace gzk
                 __syncwarp();
                 if (lane < kGroupColumns && group * kGroupColumns + lane < a.k_mapped)
                 {
-                    const uint32_t column = a.k_map[group * kGroupColumns + lane];
+                    const uint32_t column = a.mapped(group * kGroupColumns + lane);
 #pragma unroll
                     for (int p = 0; p < P; ++p)
                     {
@@ -1131,7 +1141,7 @@ namespace gzk
             const bool inject = g_inject_stall.load(std::memory_order_relaxed) != 0;
             args.wait_limit = inject ? kInjectedWaitLimit : kWaitLimit;
             args.skip_copies = inject ? 1u : 0u;
-            if (args.k_map == nullptr) args.k_mapped = args.k_count;
+            if (args.cols != nullptr && args.k_map == nullptr) args.k_mapped = args.k_count;
             const uint64_t units = static_cast<uint64_t>(args.tiles) * (mode == kIntegerGroups ? (args.k_mapped + kGroupColumns - 1) / kGroupColumns : args.k_mapped);
             uint64_t blocks = (units + (kThreads / 32) - 1) / (kThreads / 32);
             const uint64_t max_blocks = static_cast<uint64_t>(sm_count) * (blocks_per_sm_cap != 0 && blocks_per_sm_cap < static_cast<unsigned>(per_sm) ? blocks_per_sm_cap : static_cast<unsigned>(per_sm));
@@ -1157,7 +1167,7 @@ namespace gzk
         // field element - instead of a sum over stale partials.
         __global__ void __launch_bounds__(kFinishThreadsWide)
             eval_finish_kernel(const uint32_t* partial, const int* kinds, uint32_t tiles, uint32_t p_count, uint32_t k_count, Fr* out_canonical,
-                               int uniform_kind = -1, int out_montgomery = 0, const int* poison_status = nullptr)
+                               int uniform_kind = -1, int out_montgomery = 0, const int* poison_status = nullptr, uint64_t montgomery_columns = 0)
         {
             __shared__ uint32_t warp_acc[kFinishThreadsWide / 32][kAccLimbs];
             const uint32_t lane = threadIdx.x & 31;
@@ -1233,7 +1243,9 @@ namespace gzk
             // reduced = S * 2^-32 (canonical columns) -> times 2^288 via Montgomery
             // product with 2^544;  S * 2^224 (Montgomery columns) -> times 2^32 via 2^288.
             Fr fix;
-            if ((kinds != nullptr ? kinds[k] : uniform_kind) == GZK_KIND_FR_MONT)
+            // the kind of column k: from the table, the same for all, or (neither) a bit per column of a short call
+            const bool montgomery = kinds != nullptr ? kinds[k] == GZK_KIND_FR_MONT : uniform_kind >= 0 ? uniform_kind == GZK_KIND_FR_MONT : ((montgomery_columns >> k) & 1u) != 0;
+            if (montgomery)
             {
                 constexpr uint32_t c288[8] = {0xcaaf6b13u, 0x355094eau, 0x69a568efu, 0xf6b10cb3u,
                                               0x40cc3869u, 0xe2c926a6u, 0xed269aadu, 0x736a6d3bu};
@@ -1317,6 +1329,11 @@ namespace gzk
 
 using namespace gzk;
 
+namespace gzk
+{
+    int eval_status_error(gzk_ctx* ctx, int status);
+}
+
 // Shared body of gzk_eval_batch and gzk_eval_batch_range.  `rotations` are already the
 // effective ones: row c of a column meets weights[(c - rotation) mod n] of the buffer.
 // With `dest` set the results stay on the device (dest[p * k_count + k], Montgomery form when
@@ -1324,7 +1341,7 @@ using namespace gzk;
 // deferred mode.
 static int eval_batch_impl(gzk_ctx* ctx, gzk_buf* const* cols, size_t k_count, size_t len, unsigned log2n,
                            const gzk_buf* weights, const uint64_t* rotations, size_t p_count, uint8_t* out_host,
-                           Fr* dest = nullptr, bool dest_montgomery = false)
+                           Fr* dest = nullptr, bool dest_montgomery = false, bool finish = true)
 {
     const uint64_t n = 1ULL << log2n;
     if (k_count > (1u << 20)) return fail(ctx, GZK_E_INVALID, "eval_batch: too many columns");
@@ -1379,7 +1396,8 @@ static int eval_batch_impl(gzk_ctx* ctx, gzk_buf* const* cols, size_t k_count, s
 
     // device-side tables and scratch
     // column pointers, kinds, and the column indices with the field-element columns first
-    const size_t table_bytes = k_count * (sizeof(void*) + sizeof(int) + sizeof(uint32_t));
+    const bool inline_table = k_count <= kInlineColumns;
+    const size_t table_bytes = inline_table ? 0 : k_count * (sizeof(void*) + sizeof(int) + sizeof(uint32_t));
     const size_t table_padded = (table_bytes + 31) & ~static_cast<size_t>(31);
     // Host copy of the column table.  A call that reads results back ends with a synchronisation, so
     // it can stage through the context's pinned area; a call that leaves its results on the device
@@ -1390,7 +1408,7 @@ static int eval_batch_impl(gzk_ctx* ctx, gzk_buf* const* cols, size_t k_count, s
     int rc = GZK_OK;
     if (dest != nullptr)
     {
-        pageable_table.resize(table_padded);
+        pageable_table.resize(table_padded);  // empty without a table
         h_table = pageable_table.data();
     }
     else if ((rc = ensure_pinned(ctx, table_padded + p_count * k_count * 32 + 64, &h_table)) != GZK_OK)
@@ -1399,22 +1417,46 @@ static int eval_batch_impl(gzk_ctx* ctx, gzk_buf* const* cols, size_t k_count, s
     }
     void* d_table = nullptr;
     if ((rc = ensure_scratch(ctx, 0, table_padded + p_count * k_count * 32, &d_table)) != GZK_OK) return rc;
-    const void** h_ptrs = static_cast<const void**>(h_table);
-    int* h_kinds = reinterpret_cast<int*>(h_ptrs + k_count);
-    uint32_t* h_map = reinterpret_cast<uint32_t*>(h_kinds + k_count);
+    EvalArgs args{};
     uint32_t field_columns = 0;
-    for (size_t k = 0; k < k_count; ++k)
+    uint64_t montgomery_columns = 0;
+    auto is_field = [&](size_t k) { return cols[k]->kind == GZK_KIND_FR || cols[k]->kind == GZK_KIND_FR_MONT; };
+    for (size_t k = 0; k < k_count; ++k) field_columns += is_field(k) ? 1u : 0u;
+    const int* d_kinds = nullptr;
+    const uint32_t* d_map = nullptr;
+    if (inline_table)
     {
-        h_ptrs[k] = cols[k]->dptr;
-        h_kinds[k] = cols[k]->kind;
-        if (cols[k]->kind == GZK_KIND_FR || cols[k]->kind == GZK_KIND_FR_MONT) h_map[field_columns++] = static_cast<uint32_t>(k);
+        for (size_t k = 0, field = 0, other = field_columns; k < k_count; ++k)
+        {
+            args.inline_cols[k] = cols[k]->dptr;
+            args.inline_kinds[k] = static_cast<uint8_t>(cols[k]->kind);
+            args.inline_map[is_field(k) ? field++ : other++] = static_cast<uint8_t>(k);
+            if (cols[k]->kind == GZK_KIND_FR_MONT) montgomery_columns |= 1ull << k;
+        }
     }
-    for (size_t k = 0, next = field_columns; k < k_count; ++k)
-        if (cols[k]->kind != GZK_KIND_FR && cols[k]->kind != GZK_KIND_FR_MONT) h_map[next++] = static_cast<uint32_t>(k);
-    GZK_CUDA_TRY(ctx, cudaMemcpyAsync(d_table, h_table, table_bytes, cudaMemcpyHostToDevice, ctx->stream));
-    const void* const* d_ptrs = static_cast<const void* const*>(d_table);
-    const int* d_kinds = reinterpret_cast<const int*>(static_cast<const char*>(d_table) + k_count * sizeof(void*));
-    const uint32_t* d_map = reinterpret_cast<const uint32_t*>(d_kinds + k_count);
+    else
+    {
+        const void** h_ptrs = static_cast<const void**>(h_table);
+        int* h_kinds = reinterpret_cast<int*>(h_ptrs + k_count);
+        uint32_t* h_map = reinterpret_cast<uint32_t*>(h_kinds + k_count);
+        for (size_t k = 0, field = 0, other = field_columns; k < k_count; ++k)
+        {
+            h_ptrs[k] = cols[k]->dptr;
+            h_kinds[k] = cols[k]->kind;
+            h_map[is_field(k) ? field++ : other++] = static_cast<uint32_t>(k);
+        }
+        GZK_CUDA_TRY(ctx, cudaMemcpyAsync(d_table, h_table, table_bytes, cudaMemcpyHostToDevice, ctx->stream));
+        args.cols = static_cast<const void* const*>(d_table);
+        d_kinds = reinterpret_cast<const int*>(static_cast<const char*>(d_table) + k_count * sizeof(void*));
+        d_map = reinterpret_cast<const uint32_t*>(d_kinds + k_count);
+        args.kinds = d_kinds;
+    }
+    // the launch's columns: `count` of them from position `first` of the map
+    auto take_columns = [&](uint32_t first, uint32_t count) {
+        args.inline_first = first;
+        args.k_map = inline_table ? nullptr : d_map + first;
+        args.k_mapped = count;
+    };
     Fr* d_out = dest != nullptr ? dest : reinterpret_cast<Fr*>(static_cast<char*>(d_table) + table_padded);
     if (dest != nullptr && (rc = begin_call(ctx)) != GZK_OK) return rc;
 
@@ -1441,9 +1483,6 @@ static int eval_batch_impl(gzk_ctx* ctx, gzk_buf* const* cols, size_t k_count, s
         void* d_partial = nullptr;
         const size_t partial_bytes = static_cast<size_t>(tiles) * p_now * k_count * kAccLimbs * sizeof(uint32_t);
         if ((rc = ensure_scratch(ctx, 1, partial_bytes, &d_partial)) != GZK_OK) return rc;
-        EvalArgs args;
-        args.cols = d_ptrs;
-        args.kinds = d_kinds;
         args.weights = static_cast<const Fr*>(weights->dptr);
         args.len = len;
         args.mask = n - 1;
@@ -1459,8 +1498,7 @@ static int eval_batch_impl(gzk_ctx* ctx, gzk_buf* const* cols, size_t k_count, s
             if (field_columns != 0)
             {
                 LaunchScope scope(ctx, p_now == 2 ? "eval_partial_p2" : "eval_partial_p1");
-                args.k_map = d_map;
-                args.k_mapped = field_columns;
+                take_columns(0, field_columns);
                 launch_eval_partial(ctx->stream, args, static_cast<int>(p_now), ctx->sm_count, kFieldKinds);
             }
             // Small-integer columns at two evaluation points: whole groups of four on the tensor cores, and three
@@ -1474,15 +1512,13 @@ static int eval_batch_impl(gzk_ctx* ctx, gzk_buf* const* cols, size_t k_count, s
             if (grouped != 0)
             {
                 LaunchScope scope(ctx, p_now == 2 ? "eval_partial_integers_p2" : "eval_partial_integers_p1");
-                args.k_map = d_map + field_columns;
-                args.k_mapped = grouped;
+                take_columns(field_columns, grouped);
                 launch_eval_partial(ctx->stream, args, static_cast<int>(p_now), ctx->sm_count, kIntegerGroups);
             }
             if (grouped != integers)
             {
                 LaunchScope scope(ctx, p_now == 2 ? "eval_partial_integers_p2" : "eval_partial_integers_p1");
-                args.k_map = d_map + field_columns + grouped;
-                args.k_mapped = integers - grouped;
+                take_columns(field_columns + grouped, integers - grouped);
                 launch_eval_partial(ctx->stream, args, static_cast<int>(p_now), ctx->sm_count, kIntegerKinds);
             }
         }
@@ -1492,20 +1528,16 @@ static int eval_batch_impl(gzk_ctx* ctx, gzk_buf* const* cols, size_t k_count, s
             LaunchScope scope(ctx, "eval_finish");
             eval_finish_kernel<<<outs, finish_threads(tiles), 0, ctx->stream>>>(static_cast<const uint32_t*>(d_partial), d_kinds, tiles, p_now,
                                                                            static_cast<uint32_t>(k_count), d_out + p0 * k_count, -1,
-                                                                           dest != nullptr && dest_montgomery ? 1 : 0);
+                                                                           dest != nullptr && dest_montgomery ? 1 : 0, nullptr, montgomery_columns);
         }
         GZK_CUDA_TRY(ctx, cudaGetLastError());
     }
-    if (dest != nullptr) return finish_call(ctx, "eval_batch_device: invalid input");
+    if (dest != nullptr) return finish ? finish_call(ctx, "eval_batch_device: invalid input") : GZK_OK;
     GZK_CUDA_TRY(ctx, cudaMemcpyAsync(h_out, d_out, p_count * k_count * 32, cudaMemcpyDeviceToHost, ctx->stream));
     int* h_status = reinterpret_cast<int*>(h_out + p_count * k_count * 32);
     GZK_CUDA_TRY(ctx, cudaMemcpyAsync(h_status, ctx->d_status, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
     GZK_CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream));
-    if (*h_status == GZK_E_TIMEOUT)  // other codes belong to deferred calls and are reported by gzk_ctx_synchronize
-    {
-        GZK_CUDA_TRY(ctx, cudaMemsetAsync(ctx->d_status, 0, sizeof(int), ctx->stream));
-        return fail(ctx, GZK_E_TIMEOUT, "eval_batch: a bounded wait on a bulk copy gave up");
-    }
+    if ((rc = eval_status_error(ctx, *h_status)) != GZK_OK) return rc;
     std::memcpy(out_host, h_out, p_count * k_count * 32);
     return GZK_OK;
 }
@@ -1655,7 +1687,7 @@ extern "C" int gzk_eval_batch_static(int device, void* stream, const void* const
     if (cudaMemsetAsync(scratch + kStaticStatusOffset, 0, sizeof(int), s) != cudaSuccess)
         return static_fail(err, err_cap, GZK_E_CUDA, "eval_batch_static: clearing the status word failed");
 
-    EvalArgs args;
+    EvalArgs args{};
     args.cols = reinterpret_cast<const void* const*>(scratch);
     args.kinds = reinterpret_cast<const int*>(scratch + kStaticMaxColumns * sizeof(void*));
     args.weights = static_cast<const Fr*>(weights_mont);
@@ -1686,6 +1718,31 @@ extern "C" int gzk_debug_inject_eval_stall(int on)
 {
     g_inject_stall.store(on != 0 ? 1 : 0, std::memory_order_relaxed);
     return GZK_OK;
+}
+
+// The checks of gzk_eval_batch, and its sums at rotation 0 queued into `dest` (canonical); the caller reads the status
+// word after its own kernels (eval_status_error).
+namespace gzk
+{
+    int eval_batch_enqueue(gzk_ctx* ctx, gzk_buf* const* cols, size_t k_count, size_t len, unsigned log2n, const gzk_buf* weights, Fr* dest)
+    {
+        if (cols == nullptr || weights == nullptr) return fail(ctx, GZK_E_INVALID, "eval_batch: null argument");
+        if (log2n > 32) return fail(ctx, GZK_E_INVALID, "eval_batch: domain too large");
+        const uint64_t n = 1ULL << log2n;
+        if (len > n) return fail(ctx, GZK_E_INVALID, "domain evaluation backend weight size mismatch");
+        if (weights->kind != GZK_KIND_FR_MONT || weights->count < n)
+            return fail(ctx, GZK_E_INVALID, "eval_batch: weights must be a Montgomery buffer of the domain size");
+        const uint64_t zero_rotation = 0;
+        return eval_batch_impl(ctx, cols, k_count, len, log2n, weights, &zero_rotation, 1, nullptr, dest, false, false);
+    }
+
+    // `status`: the status word as read back after an evaluation
+    int eval_status_error(gzk_ctx* ctx, int status)
+    {
+        if (status != GZK_E_TIMEOUT) return GZK_OK;  // other codes belong to deferred calls and are reported by gzk_ctx_synchronize
+        GZK_CUDA_TRY(ctx, cudaMemsetAsync(ctx->d_status, 0, sizeof(int), ctx->stream));
+        return fail(ctx, GZK_E_TIMEOUT, "eval_batch: a bounded wait on a bulk copy gave up");
+    }
 }
 
 extern "C" int gzk_eval_batch(gzk_ctx* ctx, gzk_buf* const* cols, size_t k_count, size_t len, unsigned log2n,

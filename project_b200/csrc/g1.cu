@@ -374,6 +374,41 @@ namespace gzk
     }
 }
 
+namespace gzk
+{
+    // [scalars[k]] base for device scalars, canonical affine points into pinned host memory; only queued.
+    int g1_same_base_enqueue(gzk_ctx* ctx, const uint8_t base[96], const Fr* scalars, int kind, size_t count, uint8_t* out_pinned)
+    {
+        const G1Affine* table = nullptr;
+        int rc = get_base_table(ctx, base, &table);
+        if (rc != GZK_OK) return rc;
+        ColRef s;
+        s.ptr = scalars;
+        s.kind = kind;
+        if (count <= kFusedAffineLimit)
+        {
+            // a point is 96 bytes: the kernel writes them where the host reads them
+            LaunchScope scope(ctx, "g1_fixed_base_mul_affine");
+            fixed_base_mul_affine_kernel<<<static_cast<unsigned>(count), kQuadThreads, 0, ctx->stream>>>(table, s, reinterpret_cast<G1Affine*>(out_pinned), 1);
+            GZK_CUDA_TRY(ctx, cudaGetLastError());
+            return GZK_OK;
+        }
+        void* scratch = nullptr;
+        if ((rc = ensure_scratch(ctx, 1, count * (sizeof(G1Xyzz) + 2 * sizeof(Fp) + sizeof(G1Affine)), &scratch)) != GZK_OK) return rc;
+        G1Xyzz* xyzz = static_cast<G1Xyzz*>(scratch);
+        Fp* z = reinterpret_cast<Fp*>(xyzz + count);
+        G1Affine* affine = reinterpret_cast<G1Affine*>(z + 2 * count);
+        {
+            LaunchScope scope(ctx, "g1_fixed_base_mul");
+            launch_fixed_base_mul(ctx, table, s, count, xyzz);
+        }
+        GZK_CUDA_TRY(ctx, cudaGetLastError());
+        if ((rc = launch_xyzz_to_affine(ctx, xyzz, count, z, affine, true)) != GZK_OK) return rc;
+        GZK_CUDA_TRY(ctx, cudaMemcpyAsync(out_pinned, affine, count * 96, cudaMemcpyDeviceToHost, ctx->stream));
+        return GZK_OK;
+    }
+}
+
 using namespace gzk;
 
 extern "C"
@@ -412,8 +447,7 @@ extern "C"
             GZK_CUDA_TRY(ctx, cudaGetLastError());
             if ((rc = launch_xyzz_to_affine(ctx, xyzz, count, z, static_cast<G1Affine*>(out->dptr), false)) != GZK_OK) return rc;
         }
-        GZK_CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream));
-        return GZK_OK;
+        return wait_call(ctx);
     }
 
     int gzk_g1_mul_same_base(gzk_ctx* ctx, const uint8_t base[96], const uint8_t* scalars_host, size_t count, uint8_t* points_out_host)
@@ -428,37 +462,15 @@ extern "C"
             if (!canonical) return fail(ctx, GZK_E_INVALID, "g1_mul_same_base: scalar is not a canonical field element");
         }
         GZK_CUDA_TRY(ctx, cudaSetDevice(ctx->device));
-        const G1Affine* table = nullptr;
-        int rc = get_base_table(ctx, base, &table);
+        void* d_scalars = nullptr;
+        void* pinned = nullptr;
+        int rc = ensure_scratch(ctx, 3, count * sizeof(Fr), &d_scalars);
+        if (rc == GZK_OK) rc = ensure_pinned(ctx, count * 96, &pinned);
         if (rc != GZK_OK) return rc;
-        void* scratch = nullptr;
-        const size_t bytes = count * (sizeof(Fr) + sizeof(G1Xyzz) + 2 * sizeof(Fp) + sizeof(G1Affine)) + 256;
-        if ((rc = ensure_scratch(ctx, 1, bytes, &scratch)) != GZK_OK) return rc;
-        G1Xyzz* xyzz = static_cast<G1Xyzz*>(scratch);
-        Fp* z = reinterpret_cast<Fp*>(xyzz + count);
-        G1Affine* affine = reinterpret_cast<G1Affine*>(z + 2 * count);
-        Fr* d_scalars = reinterpret_cast<Fr*>(affine + count);
         GZK_CUDA_TRY(ctx, cudaMemcpyAsync(d_scalars, scalars_host, count * 32, cudaMemcpyHostToDevice, ctx->stream));
-        ColRef s;
-        s.ptr = d_scalars;
-        s.kind = GZK_KIND_FR;
-        if (count <= kFusedAffineLimit)
-        {
-            LaunchScope scope(ctx, "g1_fixed_base_mul_affine");
-            fixed_base_mul_affine_kernel<<<static_cast<unsigned>(count), kQuadThreads, 0, ctx->stream>>>(table, s, affine, 1);
-            GZK_CUDA_TRY(ctx, cudaGetLastError());
-        }
-        else
-        {
-            {
-                LaunchScope scope(ctx, "g1_fixed_base_mul");
-                launch_fixed_base_mul(ctx, table, s, count, xyzz);
-            }
-            GZK_CUDA_TRY(ctx, cudaGetLastError());
-            if ((rc = launch_xyzz_to_affine(ctx, xyzz, count, z, affine, true)) != GZK_OK) return rc;
-        }
-        GZK_CUDA_TRY(ctx, cudaMemcpyAsync(points_out_host, affine, count * 96, cudaMemcpyDeviceToHost, ctx->stream));
+        if ((rc = g1_same_base_enqueue(ctx, base, static_cast<const Fr*>(d_scalars), GZK_KIND_FR, count, static_cast<uint8_t*>(pinned))) != GZK_OK) return rc;
         GZK_CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream));
+        std::memcpy(points_out_host, pinned, count * 96);
         return GZK_OK;
     }
 

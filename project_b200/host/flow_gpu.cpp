@@ -97,6 +97,15 @@ namespace
             check(gzk_buf_download(ctx_, raw(col), offset, host, count));
             downloaded_bytes += count * element_bytes(col->kind);
         }
+        void download_elements(const std::vector<ColP>& cols, const std::vector<std::uint64_t>& indices, Fe* out) override
+        {
+            std::vector<const gzk_buf*> bufs;
+            for (const auto& c : cols) bufs.push_back(raw(c));
+            std::vector<std::uint8_t> bytes(32 * cols.size());
+            check(gzk_buf_download_elements(ctx_, bufs.data(), indices.data(), bufs.size(), bytes.data()));
+            for (std::size_t i = 0; i < cols.size(); ++i) std::memcpy(out[i].data(), bytes.data() + 32 * i, 32);
+            downloaded_bytes += bytes.size();
+        }
         void zero(const ColP& col) override { check(gzk_buf_zero(ctx_, raw(col))); }
         void copy_block(const ColP& src, std::size_t so, std::size_t ss, const ColP& dst, std::size_t d_o, std::size_t ds, std::size_t rows,
                         std::size_t width) override

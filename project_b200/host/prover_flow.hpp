@@ -107,6 +107,11 @@ namespace gatzk_flow
         virtual ColP alloc(int kind, std::size_t count) = 0;
         virtual void upload(const ColP& col, const void* host, std::size_t count) = 0;
         virtual void download(const ColP& col, std::size_t offset, std::size_t count, void* host) = 0;
+        // element indices[i] of field-element column cols[i]; one wait where the backend can
+        virtual void download_elements(const std::vector<ColP>& cols, const std::vector<std::uint64_t>& indices, Fe* out)
+        {
+            for (std::size_t i = 0; i < cols.size(); ++i) download(cols[i], indices[i], 1, out + i);
+        }
         virtual void zero(const ColP& col) = 0;
         virtual void copy_block(const ColP& src, std::size_t src_offset, std::size_t src_stride, const ColP& dst, std::size_t dst_offset,
                                 std::size_t dst_stride, std::size_t rows, std::size_t width) = 0;
@@ -579,12 +584,16 @@ namespace gatzk_flow
         void resolve_totals()
         {
             flush_scans();
+            std::vector<ColP> cols;
+            std::vector<std::uint64_t> indices;
             for (const auto& p : pending_totals_)
             {
-                Fe v{};
-                be_.download(p.column, p.index, 1, v.data());
-                witness_scalars_.push_back({p.name, v});
+                cols.push_back(p.column);
+                indices.push_back(p.index);
             }
+            std::vector<Fe> values(cols.size());
+            be_.download_elements(cols, indices, values.data());
+            for (std::size_t i = 0; i < values.size(); ++i) witness_scalars_.push_back({pending_totals_[i].name, values[i]});
             pending_totals_.clear();
         }
 
@@ -1083,12 +1092,27 @@ namespace gatzk_flow
         const bool host_fix = !tail_items.empty() || !derived_items.empty();
         if (host_fix)
         {
+            // the evaluations, those of the columns of ones and the tails in one read-back
             std::vector<Fe> ones_host(ones_slot.size());
-            be_.download(scalars, 0, items.size(), evals_by_slot.data());
-            if (!tail_items.empty()) be_.download(ones_out, 0, ones_host.size(), ones_host.data());
+            {
+                std::vector<ColP> cols;
+                std::vector<std::uint64_t> indices;
+                auto want = [&](const ColP& col, std::size_t index) {
+                    cols.push_back(col);
+                    indices.push_back(index);
+                };
+                for (std::size_t i = 0; i < items.size(); ++i) want(scalars, i);
+                for (std::size_t i = 0; i < ones_host.size(); ++i) want(ones_out, i);
+                for (const auto i : tail_items) want(items[i].col, items[i].length - 1);
+                std::vector<Fe> values(cols.size());
+                be_.download_elements(cols, indices, values.data());
+                auto next_value = values.begin();
+                for (auto& v : evals_by_slot) v = *next_value++;
+                for (auto& v : ones_host) v = *next_value++;
+                for (const auto i : tail_items) tails[i] = *next_value++;
+            }
             for (const auto i : tail_items)
             {
-                be_.download(items[i].col, items[i].length - 1, 1, &tails[i]);
                 const Fe rest = sub(fe_u64(1), ones_host[ones_slot.at({items[i].domain, items[i].length})]);
                 evals_by_slot[slot[i]] = add(evals_by_slot[slot[i]], mul(tails[i], rest));
             }
