@@ -103,7 +103,8 @@ namespace gzk
     // its own value, so a step costs two multiplications and nothing is undone afterwards; the warp products
     // go through the same butterfly in every warp, which leaves warp 0 with the total it inverts (a chain of
     // 10 + 5 multiplications around the inversion at 256 threads; a prefix and a suffix scan with the warp
-    // products in sequence take 10 + 16 + 5).
+    // products in sequence take 10 + 16 + 5).  Which warp inverts follows from the block's number: a warp's number
+    // decides the scheduler it runs on, and with warp 0 everywhere the inversions of all CTAs of an SM would share one.
     template <int THREADS>
     __device__ __forceinline__ Fr block_batch_invert(const Fr& mine, BatchInvertShared<THREADS>& sh, bool* zero)
     {
@@ -136,7 +137,7 @@ namespace gzk
             others = mul(others, shfl_fr_idx(warp_others, warp));
         }
         *zero = product.is_zero();
-        if (warp == 0)
+        if (warp == static_cast<int>(((blockIdx.x + blockIdx.y) * 0x9e3779b1u >> 16) & (W - 1)))
         {
             const Fr inverse = inv_quad<FrCfg>(product);
             if (lane == 0) sh.inverse = inverse;

@@ -62,6 +62,17 @@ namespace gzk
             __device__ __forceinline__ int kind(uint32_t k) const { return cols != nullptr ? kinds[k] : static_cast<int>(inline_kinds[k]); }
             __device__ __forceinline__ uint32_t mapped(uint32_t i) const { return cols == nullptr ? inline_map[inline_first + i] : k_map != nullptr ? k_map[i] : i; }
         };
+        // The value, kept in its register: an indexed read of a launch parameter counts as cheap, and the compiler would
+        // repeat it inside the loop over the rows (201 -> 230 us for eight columns of 2.5 M rows at two points).
+        template <typename T>
+        __device__ __forceinline__ T held(T v)
+        {
+            if constexpr (sizeof(T) == 8)
+                asm volatile("" : "+l"(v));
+            else
+                asm volatile("" : "+r"(v));
+            return v;
+        }
         // Which columns a launch takes.  Field-element columns run through the shared-memory ring and the tensor
         // cores; small-integer columns in groups of four through a tensor-core kernel of their own
         // (kIntegerGroups), the ones left over through plain loads and the integer pipe (kIntegerKinds: many resident
@@ -263,7 +274,7 @@ namespace gzk
                 const uint32_t tile = static_cast<uint32_t>(u / a.k_mapped);
                 const uint32_t slot_of_k = static_cast<uint32_t>(u - static_cast<uint64_t>(tile) * a.k_mapped);
                 const uint32_t k = a.mapped(slot_of_k);
-                const void* col = a.column(k);
+                const void* col = held(a.column(k));
                 const int kind = a.kind(k);
                 const uint64_t c_begin = static_cast<uint64_t>(tile) * a.tile_rows;
                 const uint64_t c_end = c_begin + a.tile_rows < a.len ? c_begin + a.tile_rows : a.len;
@@ -655,8 +666,8 @@ namespace gzk
                     const uint32_t slot = group * kGroupColumns + c;
                     const bool there = slot < a.k_mapped;
                     const uint32_t k = there ? a.mapped(slot) : 0;
-                    column_of[c] = there ? static_cast<const unsigned char*>(a.column(k)) : nullptr;
-                    wide_of[c] = there && a.kind(k) == GZK_KIND_I64;
+                    column_of[c] = held(there ? static_cast<const unsigned char*>(a.column(k)) : nullptr);
+                    wide_of[c] = held(there && a.kind(k) == GZK_KIND_I64 ? 1 : 0) != 0;
                 }
                 const bool present = group * kGroupColumns + my_column < a.k_mapped;
                 bool wide = false;
