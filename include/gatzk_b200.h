@@ -386,6 +386,10 @@ int gzk_fh_public_eval_rotated(gzk_ctx* ctx, const gzk_buf* features, size_t row
  * returns both the scalars p_k(tau) (Commitment::tau_evaluation) and the points. */
 int gzk_g1_mul_same_base(gzk_ctx* ctx, const uint8_t base[96], const uint8_t* scalars_host, size_t count, uint8_t* points_out_host);
 int gzk_g1_fixed_base_mul(gzk_ctx* ctx, const uint8_t base[96], const gzk_buf* scalars, size_t count, gzk_buf* out);
+/* the same points straight to the host, with the scalars they belong to (canonical; NULL: not wanted): the end of a
+ * commit barrier in one wait */
+int gzk_g1_fixed_base_mul_download(gzk_ctx* ctx, const uint8_t base[96], const gzk_buf* scalars, size_t count, uint8_t* scalars_out,
+                                   uint8_t* points_out);
 int gzk_commit_batch(gzk_ctx* ctx, gzk_buf* const* cols, size_t k_count, size_t len, unsigned log2n, const gzk_buf* weights_tau,
                      const uint8_t base[96], uint8_t* tau_evals_out, uint8_t* points_out);
 

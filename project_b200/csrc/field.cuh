@@ -279,29 +279,31 @@ namespace gzk
             }
         }
 
-        // Divides the running value by 2^32 where nothing is added to it (see mont_row).
+        // Divides the running value by 2^32 where no product is added to it (see mont_row); `in` joins at limb N - 1.
         template <typename Cfg>
-        GZK_HD void shift_row(uint32_t* P, uint32_t* Q)
+        GZK_HD void shift_row(uint32_t* P, uint32_t* Q, uint32_t in = 0)
         {
             constexpr int N = Cfg::N;
             P[0] = mp::add_cc(P[0], Q[1]);
 #pragma unroll
-            for (int j = 0; j < N - 1; ++j) Q[j] = mp::addc_cc(Q[j + 2], 0);
+            for (int j = 0; j < N - 2; ++j) Q[j] = mp::addc_cc(Q[j + 2], 0);
+            Q[N - 2] = mp::addc_cc(Q[N], in);
             Q[N - 1] = mp::addc(0, 0);
             Q[N] = 0;
             P[N] = 0;
         }
 
-        // The value after the last row: Y is even-aligned (limb 0 zero) and X odd-aligned, (Y >> 32) + X < 2*modulus.
+        // The value after the last row: Y is even-aligned (limb 0 zero) and X odd-aligned,
+        // (Y >> 32) + X + in 2^(32 (N-1)) < 2*modulus.
         template <typename Cfg>
-        GZK_HD Fe<Cfg> join_rows(const uint32_t* X, const uint32_t* Y)
+        GZK_HD Fe<Cfg> join_rows(const uint32_t* X, const uint32_t* Y, uint32_t in = 0)
         {
             constexpr int N = Cfg::N;
             Fe<Cfg> s;
             s.l[0] = mp::add_cc(Y[1], X[0]);
 #pragma unroll
             for (int k = 1; k < N - 1; ++k) s.l[k] = mp::addc_cc(Y[k + 1], X[k]);
-            s.l[N - 1] = mp::addc(Y[N], X[N - 1]);
+            s.l[N - 1] = mp::addc(Y[N], X[N - 1]) + in;
             return reduce_once(s);
         }
 
@@ -936,38 +938,34 @@ namespace gzk
     }
 
     // Montgomery reduction of a wide integer T (N + ROWS limbs, T < modulus *
-    // 2^(32*ROWS)): returns T * 2^(-32*ROWS) mod modulus, fully reduced.  Used
-    // once per accumulated inner product, so it favours clarity over speed.
+    // 2^(32*ROWS)): returns T * 2^(-32*ROWS) mod modulus, fully reduced.  The rows of mul() on a window of N
+    // limbs, which the next limb of T joins at the top after every row.
     template <typename Cfg, int ROWS>
-    GZK_HD Fe<Cfg> redc_wide(const uint32_t* T_in)
+    GZK_HD Fe<Cfg> redc_wide(const uint32_t* T)
     {
         constexpr int N = Cfg::N;
-        constexpr int L = N + ROWS + 1;
-        uint32_t T[L];
+        uint32_t X[N + 1], Y[N + 1];
 #pragma unroll
-        for (int k = 0; k < L - 1; ++k) T[k] = T_in[k];
-        T[L - 1] = 0;
-#pragma unroll
-        for (int i = 0; i < ROWS; ++i)
+        for (int j = 0; j < N; ++j)
         {
-            const uint32_t m = mp::mul_lo(T[i], Cfg::INV);
-            // low halves
-            T[i] = mp::mad_lo_cc(m, Cfg::mod(0), T[i]);
-#pragma unroll
-            for (int j = 1; j < N; ++j) T[i + j] = mp::madc_lo_cc(m, Cfg::mod(j), T[i + j]);
-#pragma unroll
-            for (int k = i + N; k < L; ++k) T[k] = mp::addc_cc(T[k], 0);
-            // high halves
-            T[i + 1] = mp::mad_hi_cc(m, Cfg::mod(0), T[i + 1]);
-#pragma unroll
-            for (int j = 1; j < N; ++j) T[i + j + 1] = mp::madc_hi_cc(m, Cfg::mod(j), T[i + j + 1]);
-#pragma unroll
-            for (int k = i + N + 1; k < L; ++k) T[k] = mp::addc_cc(T[k], 0);
+            X[j] = T[j];
+            Y[j] = 0;
         }
-        Fe<Cfg> s;
+        X[N] = 0;
+        Y[N] = 0;
+        detail::reduce_row<Cfg>(X, Y);
 #pragma unroll
-        for (int k = 0; k < N; ++k) s.l[k] = T[ROWS + k];
-        return reduce_once(s);
+        for (int i = 1; i < ROWS; i += 2)
+        {
+            detail::shift_row<Cfg>(Y, X, T[N + i - 1]);
+            detail::reduce_row<Cfg>(Y, X);
+            if (i + 1 < ROWS)
+            {
+                detail::shift_row<Cfg>(X, Y, T[N + i]);
+                detail::reduce_row<Cfg>(X, Y);
+            }
+        }
+        return ROWS % 2 == 0 ? detail::join_rows<Cfg>(X, Y, T[N + ROWS - 1]) : detail::join_rows<Cfg>(Y, X, T[N + ROWS - 1]);
     }
 
     // Unreduced accumulator for sums of 8x8-limb products (inner products of Fr

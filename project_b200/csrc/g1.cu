@@ -450,6 +450,28 @@ extern "C"
         return wait_call(ctx);
     }
 
+    int gzk_g1_fixed_base_mul_download(gzk_ctx* ctx, const uint8_t base[96], const gzk_buf* scalars, size_t count, uint8_t* scalars_out, uint8_t* points_out)
+    {
+        if (ctx == nullptr) return GZK_E_INVALID;
+        if (count == 0) return GZK_OK;
+        if (base == nullptr || scalars == nullptr || points_out == nullptr) return fail(ctx, GZK_E_INVALID, "g1_fixed_base_mul: null argument");
+        if ((scalars->kind != GZK_KIND_FR && scalars->kind != GZK_KIND_FR_MONT) || scalars->count < count)
+            return fail(ctx, GZK_E_INVALID, "g1_fixed_base_mul: scalars must be an FR or FR_MONT buffer");
+        GZK_CUDA_TRY(ctx, cudaSetDevice(ctx->device));
+        void* pinned = nullptr;
+        int rc = ensure_pinned(ctx, count * (96 + sizeof(Fr)), &pinned);
+        if (rc != GZK_OK) return rc;
+        uint8_t* h_points = static_cast<uint8_t*>(pinned);
+        const bool copied = scalars_out != nullptr && scalars->kind == GZK_KIND_FR;
+        if (copied) GZK_CUDA_TRY(ctx, cudaMemcpyAsync(h_points + 96 * count, scalars->dptr, count * sizeof(Fr), cudaMemcpyDeviceToHost, ctx->stream));
+        if ((rc = g1_same_base_enqueue(ctx, base, static_cast<const Fr*>(scalars->dptr), scalars->kind, count, h_points)) != GZK_OK) return rc;
+        GZK_CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream));
+        std::memcpy(points_out, h_points, count * 96);
+        if (copied) std::memcpy(scalars_out, h_points + 96 * count, count * sizeof(Fr));
+        if (scalars_out != nullptr && !copied) return gzk_buf_download(ctx, scalars, 0, scalars_out, count);
+        return GZK_OK;
+    }
+
     int gzk_g1_mul_same_base(gzk_ctx* ctx, const uint8_t base[96], const uint8_t* scalars_host, size_t count, uint8_t* points_out_host)
     {
         if (ctx == nullptr) return GZK_E_INVALID;

@@ -320,6 +320,17 @@ namespace
         {
             check(gzk_g1_fixed_base_mul(ctx_, base.data(), raw(scalars), count, raw(out_points)));
         }
+        void g1_fixed_base_download(const G1& base, const ColP& scalars, std::size_t count, Fe* values, G1* points) override
+        {
+            std::vector<std::uint8_t> bytes(values != nullptr ? 32 * count : 0), point_bytes(96 * count);
+            check(gzk_g1_fixed_base_mul_download(ctx_, base.data(), raw(scalars), count, values != nullptr ? bytes.data() : nullptr, point_bytes.data()));
+            for (std::size_t i = 0; i < count; ++i)
+            {
+                if (values != nullptr) std::memcpy(values[i].data(), bytes.data() + 32 * i, 32);
+                std::memcpy(points[i].data(), point_bytes.data() + 96 * i, 96);
+            }
+            downloaded_bytes += bytes.size() + point_bytes.size();
+        }
         void fh_public_eval(const ColP& features, std::size_t rows, std::size_t fc, const ColP& abs_ids, const ColP& weights, unsigned log2n,
                             std::uint64_t rotation, Fe out[5]) override
         {

@@ -180,6 +180,14 @@ namespace gatzk_flow
                                  const std::vector<std::uint64_t>& rotations, const ColP& out, std::size_t out_offset) = 0;
         virtual void horner_device(const ColP& matrix, std::size_t rows, std::size_t cols, const Fe& x, const ColP& out, std::size_t out_offset) = 0;
         virtual void g1_fixed_base(const G1& base, const ColP& scalars, std::size_t count, const ColP& out_points) = 0;
+        // the points [scalar] base on the host, and the scalars themselves where `values` is given
+        virtual void g1_fixed_base_download(const G1& base, const ColP& scalars, std::size_t count, Fe* values, G1* points)
+        {
+            const ColP out = alloc(kG1, count);
+            g1_fixed_base(base, scalars, count, out);
+            if (values != nullptr) download(scalars, 0, count, values);
+            download(out, 0, count, points);
+        }
         // weights: those of the whole 2^log2n domain at a point z; rotation r gives the sums at omega^r * z
         virtual void fh_public_eval(const ColP& features, std::size_t rows, std::size_t feature_count, const ColP& abs_ids, const ColP& weights,
                                     unsigned log2n, std::uint64_t rotation, Fe out[5]) = 0;
@@ -1139,11 +1147,8 @@ namespace gatzk_flow
             }
             scalars = upload_fe(evals_by_slot, items.size());
         }
-        const ColP points = be_.alloc(kG1, items.size());
-        be_.g1_fixed_base(in_.generator, scalars, items.size(), points);
         std::vector<G1> pts(items.size()), pts_by_slot(items.size());
-        if (!host_fix) be_.download(scalars, 0, items.size(), evals_by_slot.data());
-        be_.download(points, 0, items.size(), pts_by_slot.data());
+        be_.g1_fixed_base_download(in_.generator, scalars, items.size(), host_fix ? nullptr : evals_by_slot.data(), pts_by_slot.data());
         for (std::size_t i = 0; i < items.size(); ++i)
         {
             evals[i] = evals_by_slot[slot[i]];

@@ -369,10 +369,8 @@ namespace gatzk_flow
             std::vector<Fe> scalars;
             for (const auto& item : lazy) scalars.push_back(item.second);
             const ColP s = upload_fe(scalars, scalars.size());
-            const ColP p = be_.alloc(kG1, scalars.size());
-            be_.g1_fixed_base(in_.generator, s, scalars.size(), p);
             std::vector<G1> pts(scalars.size());
-            be_.download(p, 0, scalars.size(), pts.data());
+            be_.g1_fixed_base_download(in_.generator, s, scalars.size(), nullptr, pts.data());
             for (std::size_t i = 0; i < lazy.size(); ++i)
             {
                 commitments_[lazy[i].first] = Commitment{pts[i], lazy[i].second};
@@ -670,9 +668,7 @@ namespace gatzk_flow
         std::vector<G1> quotient_points(7);
         {
             const ColP s = upload_fe(quotient_values, 7);
-            const ColP p = be_.alloc(kG1, 7);
-            be_.g1_fixed_base(in_.generator, s, 7, p);
-            be_.download(p, 0, 7, quotient_points.data());
+            be_.g1_fixed_base_download(in_.generator, s, 7, nullptr, quotient_points.data());
         }
         for (int di = 0; di < 7; ++di) t.absorb_commitment(std::string("t_") + kBundles[di], quotient_points[di]);
         std::map<std::string, Fe> z, v;
@@ -789,9 +785,7 @@ namespace gatzk_flow
         std::vector<G1> pts(all.size());
         {
             const ColP s = upload_fe(all, all.size());
-            const ColP p = be_.alloc(kG1, all.size());
-            be_.g1_fixed_base(in_.generator, s, all.size(), p);
-            be_.download(p, 0, all.size(), pts.data());
+            be_.g1_fixed_base_download(in_.generator, s, all.size(), nullptr, pts.data());
         }
         for (int di = 0; di < 7; ++di) proof_.domain_openings[di].second.witness = point_bytes(pts[di]);
         proof_.external_witness = point_bytes(pts[7]);
