@@ -93,6 +93,8 @@ struct gzk_ctx
     int* h_status = nullptr;  // pinned copy of it, read at the end of a call that waits
     // zero between the kernels of the stream: counts the CTAs of a launch that have left their partial result
     uint32_t* arrival_counter() const { return reinterpret_cast<uint32_t*>(d_status) + 8; }
+    uint32_t* column_counters() const { return reinterpret_cast<uint32_t*>(d_status) + 16; }  // 64 of them, one per column of a short evaluation
+    static constexpr size_t kStatusBytes = (16 + 64) * sizeof(uint32_t);
     // pinned ring for the small uploads of deferred mode: the data is copied into a slot and the
     // call returns without waiting; a slot is reused once the copy that read it has completed
     static constexpr int kUploadSlots = 16;

@@ -1173,6 +1173,154 @@ namespace gzk
         constexpr int kFinishThreadsWide = 512;  // more
         constexpr int kFinishGroup = 4;
         inline unsigned finish_threads(uint32_t tiles) { return tiles > 1024 ? kFinishThreadsWide : kFinishThreads; }
+        // The field value of a 17-limb sum: acc = 2^256 * S (canonical columns) or 2^512 * S (Montgomery columns), S the
+        // true sum; 9 reduction rows divide by 2^288, which leaves S * 2^-32 (times 2^288 via the Montgomery product with
+        // 2^544) or S * 2^224 (times 2^32 via 2^288).
+        __device__ __forceinline__ Fr eval_value(const uint32_t* acc, bool montgomery_column, bool out_montgomery)
+        {
+            const Fr reduced = redc_wide<FrCfg, 9>(acc);
+            Fr fix;
+            if (montgomery_column)
+            {
+                constexpr uint32_t c288[8] = {0xcaaf6b13u, 0x355094eau, 0x69a568efu, 0xf6b10cb3u,
+                                              0x40cc3869u, 0xe2c926a6u, 0xed269aadu, 0x736a6d3bu};
+#pragma unroll
+                for (int i = 0; i < 8; ++i) fix.l[i] = c288[i];
+            }
+            else
+            {
+                fix = fr_const_2_544();
+            }
+            const Fr mont = mul(reduced, fix);  // Montgomery form of S
+            return out_montgomery ? mont : from_mont(mont);
+        }
+        __device__ __forceinline__ void warp_sum_limbs(uint32_t* acc)
+        {
+#pragma unroll 1
+            for (int offset = 16; offset > 0; offset >>= 1)
+            {
+                uint32_t other[kAccLimbs];
+#pragma unroll
+                for (int i = 0; i < kAccLimbs; ++i) other[i] = __shfl_down_sync(0xffffffffu, acc[i], offset);
+                acc_add<kAccLimbs, kAccLimbs>(acc, other);
+            }
+        }
+
+        // A short call in ONE launch: CTA (column, slice of the rows) on the integer pipe, the CTA of a column that
+        // arrives last (nobody waits) adds the slices up and reduces.  Most evaluations of a proof are a few columns
+        // of a few thousand rows, where the tensor-core kernels (one launch per kind of column, whose shared-memory
+        // rings and folds want long units) and the finishing launch each cost more than the products: a commit of
+        // eight field-element and sixteen integer columns of 19717 rows spent 20 us on them and takes 13 now (call 111 -> 106 us;
+        // proof of a 1500-node graph 9.65 -> 9.11 ms).
+        constexpr uint32_t kShortSliceRows = 2048;
+        constexpr uint32_t kShortSlices = 64;
+        constexpr uint64_t kShortProducts = 40ull << 20;  // limb products of a short call: about 5 us of the integer pipe
+        struct ShortEval
+        {
+            uint32_t slices, out_montgomery;
+            uint32_t* arrived;  // one word per column, zero between the launches
+            Fr* out;
+        };
+        template <int P>
+        __global__ void __launch_bounds__(kFinishThreads) eval_short_kernel(const __grid_constant__ EvalArgs a, const __grid_constant__ ShortEval e)
+        {
+            constexpr int kShortWarps = kFinishThreads / 32;
+            __shared__ uint32_t warp_acc[P][kShortWarps][kAccLimbs];
+            __shared__ bool last;
+            const uint32_t k = blockIdx.x, slice = blockIdx.y, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+            const void* col = held(a.column(k));
+            const int kind = held(a.kind(k));
+            const uint64_t begin = static_cast<uint64_t>(slice) * kShortSliceRows;
+            const uint64_t end = begin + kShortSliceRows < a.len ? begin + kShortSliceRows : a.len;
+            WideAcc acc[P];
+#pragma unroll
+            for (int p = 0; p < P; ++p) acc[p].clear();
+            if (kind == GZK_KIND_FR || kind == GZK_KIND_FR_MONT)
+            {
+                for (uint64_t c = begin + threadIdx.x; c < end; c += kFinishThreads)
+                {
+                    const Fr x = load_fr(static_cast<const Fr*>(col) + c);
+#pragma unroll
+                    for (int p = 0; p < P; ++p)
+                    {
+                        const Fr w = load_fr(a.weights + ((c - a.rot[p]) & a.mask));
+                        acc[p].template mac<8>(w.l, x.l);
+                    }
+                }
+            }
+            else
+            {
+                for (uint64_t c = begin + threadIdx.x; c < end; c += kFinishThreads)
+                {
+                    const long long v = kind == GZK_KIND_U32 ? static_cast<long long>(__ldg(static_cast<const uint32_t*>(col) + c)) : __ldg(static_cast<const long long*>(col) + c);
+                    const unsigned long long mag = v < 0 ? 0ULL - static_cast<unsigned long long>(v) : static_cast<unsigned long long>(v);
+                    const uint32_t f[2] = {static_cast<uint32_t>(mag), static_cast<uint32_t>(mag >> 32)};
+#pragma unroll
+                    for (int p = 0; p < P; ++p)
+                    {
+                        Fr w = load_fr(a.weights + ((c - a.rot[p]) & a.mask));
+                        if (v < 0) w = sub(Fr::zero(), w);
+                        if (f[1] == 0)
+                            acc[p].template mac<1>(w.l, f);
+                        else
+                            acc[p].template mac<2>(w.l, f);
+                    }
+                }
+            }
+#pragma unroll
+            for (int p = 0; p < P; ++p)
+            {
+                uint32_t sum[kAccLimbs];
+                acc[p].fold(sum);
+                warp_sum_limbs(sum);
+                if (lane == 0)
+                {
+#pragma unroll
+                    for (int i = 0; i < kAccLimbs; ++i) warp_acc[p][warp][i] = sum[i];
+                }
+            }
+            __syncthreads();
+            // warp p finishes point p
+            uint32_t sum[kAccLimbs];
+            if (warp < P)
+            {
+#pragma unroll
+                for (int i = 0; i < kAccLimbs; ++i) sum[i] = lane < kShortWarps ? warp_acc[warp][lane][i] : 0u;
+                warp_sum_limbs(sum);
+            }
+            if (e.slices > 1)
+            {
+                if (warp < P && lane == 0)
+                {
+                    uint32_t* dst = a.partial + ((static_cast<uint64_t>(slice) * P + warp) * a.k_count + k) * kAccLimbs;
+#pragma unroll
+                    for (int i = 0; i < kAccLimbs; ++i) dst[i] = sum[i];
+                    __threadfence();
+                }
+                __syncthreads();
+                if (threadIdx.x == 0) last = atomicAdd(e.arrived + k, 1u) + 1 == e.slices;
+                __syncthreads();
+                if (!last) return;
+                __threadfence();
+                if (threadIdx.x == 0) e.arrived[k] = 0;  // for the next call
+                if (warp < P)
+                {
+#pragma unroll
+                    for (int i = 0; i < kAccLimbs; ++i) sum[i] = 0;
+                    for (uint32_t s2 = lane; s2 < e.slices; s2 += 32)
+                    {
+                        const uint32_t* src = a.partial + ((static_cast<uint64_t>(s2) * P + warp) * a.k_count + k) * kAccLimbs;
+                        uint32_t t[kAccLimbs];
+#pragma unroll
+                        for (int i = 0; i < kAccLimbs; ++i) t[i] = __ldcg(src + i);
+                        acc_add<kAccLimbs, kAccLimbs>(sum, t);
+                    }
+                    warp_sum_limbs(sum);
+                }
+            }
+            if (warp < P && lane == 0) store_fr(e.out + static_cast<size_t>(warp) * a.k_count + k, eval_value(sum, kind == GZK_KIND_FR_MONT, e.out_montgomery != 0));
+        }
+
         // `poison_status`: when given and raised (a bounded wait of the partial kernel gave up, so some
         // partial sums were never written), every output becomes 32 bytes of 0xFF - not a canonical
         // field element - instead of a sum over stale partials.
@@ -1248,27 +1396,9 @@ namespace gzk
             for (int i = 0; i < kAccLimbs; ++i) acc[i] = lane < (threads >> 5) ? warp_acc[lane][i] : 0u;
             warp_sum();
             if (lane != 0) return;
-            // acc = 2^256 * S (canonical columns) or 2^512 * S (Montgomery columns), S the
-            // true sum; 9 reduction rows divide by 2^288.
-            const Fr reduced = redc_wide<FrCfg, 9>(acc);
-            // reduced = S * 2^-32 (canonical columns) -> times 2^288 via Montgomery
-            // product with 2^544;  S * 2^224 (Montgomery columns) -> times 2^32 via 2^288.
-            Fr fix;
             // the kind of column k: from the table, the same for all, or (neither) a bit per column of a short call
             const bool montgomery = kinds != nullptr ? kinds[k] == GZK_KIND_FR_MONT : uniform_kind >= 0 ? uniform_kind == GZK_KIND_FR_MONT : ((montgomery_columns >> k) & 1u) != 0;
-            if (montgomery)
-            {
-                constexpr uint32_t c288[8] = {0xcaaf6b13u, 0x355094eau, 0x69a568efu, 0xf6b10cb3u,
-                                              0x40cc3869u, 0xe2c926a6u, 0xed269aadu, 0x736a6d3bu};
-#pragma unroll
-                for (int i = 0; i < 8; ++i) fix.l[i] = c288[i];
-            }
-            else
-            {
-                fix = fr_const_2_544();
-            }
-            const Fr mont = mul(reduced, fix);  // Montgomery form of S
-            store_fr(out_canonical + idx, out_montgomery ? mont : from_mont(mont));
+            store_fr(out_canonical + idx, eval_value(acc, montgomery, out_montgomery != 0));
         }
     }
 }
@@ -1488,11 +1618,15 @@ static int eval_batch_impl(gzk_ctx* ctx, gzk_buf* const* cols, size_t k_count, s
         ctx->eval_limb_products += limbs * p_count;
         ctx->eval_terms += static_cast<uint64_t>(len) * k_count * p_count;
     }
+    const uint64_t short_slices = len == 0 ? 1 : (len + kShortSliceRows - 1) / kShortSliceRows;
+    const uint64_t products = static_cast<uint64_t>(len) * (64 * field_columns + 8 * (k_count - field_columns)) * (p_count >= 2 ? 2 : 1);
+    // (the stall injection wants the bounded waits of the long kernels)
+    const bool short_call = inline_table && short_slices <= kShortSlices && products <= kShortProducts && g_inject_stall.load(std::memory_order_relaxed) == 0;
     for (size_t p0 = 0; p0 < p_count; p0 += 2)
     {
         const uint32_t p_now = p_count - p0 >= 2 ? 2 : 1;
         void* d_partial = nullptr;
-        const size_t partial_bytes = static_cast<size_t>(tiles) * p_now * k_count * kAccLimbs * sizeof(uint32_t);
+        const size_t partial_bytes = static_cast<size_t>(short_call ? short_slices : tiles) * p_now * k_count * kAccLimbs * sizeof(uint32_t);
         if ((rc = ensure_scratch(ctx, 1, partial_bytes, &d_partial)) != GZK_OK) return rc;
         args.weights = static_cast<const Fr*>(weights->dptr);
         args.len = len;
@@ -1504,6 +1638,22 @@ static int eval_batch_impl(gzk_ctx* ctx, gzk_buf* const* cols, size_t k_count, s
         args.rot[1] = p_now == 2 ? rotations[p0 + 1] : 0;
         args.partial = static_cast<uint32_t*>(d_partial);
         args.status = ctx->d_status;
+        if (short_call)
+        {
+            ShortEval e;
+            e.slices = static_cast<uint32_t>(short_slices);
+            e.out_montgomery = dest != nullptr && dest_montgomery ? 1u : 0u;
+            e.arrived = ctx->column_counters();
+            e.out = d_out + p0 * k_count;
+            const dim3 grid(static_cast<unsigned>(k_count), static_cast<unsigned>(short_slices));
+            LaunchScope scope(ctx, "eval_short");
+            if (p_now == 2)
+                eval_short_kernel<2><<<grid, kFinishThreads, 0, ctx->stream>>>(args, e);
+            else
+                eval_short_kernel<1><<<grid, kFinishThreads, 0, ctx->stream>>>(args, e);
+            GZK_CUDA_TRY(ctx, cudaGetLastError());
+            continue;
+        }
         {
             // one launch per kind of column present, over the same partial buffer
             if (field_columns != 0)

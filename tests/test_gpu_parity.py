@@ -373,3 +373,30 @@ def test_eval_long_units_fold_their_byte_products_in_time(be):
     integer_column.free()
     field_column.free()
     w.free()
+
+
+@pytest.mark.parametrize("rows", [0, 1, 255, 2047, 2048, 2049, 6000, 131072, 131073])  # one slice, several, the most a short call has, one more
+@pytest.mark.parametrize("points", [1, 2, 3])
+def test_short_evaluation_slices(be, rows, points):
+    """Calls of few rows take the one-launch kernel; longer ones and more than 64 columns the kernels by kind."""
+    from project_b200 import KIND_FR, KIND_FR_MONT, KIND_I64, KIND_U32
+
+    log2n = max(2, (max(rows, 1) - 1).bit_length())
+    n = 1 << log2n
+    rng = np.random.default_rng(rows + points)
+    w = be.bary_weights(log2n, fr_array([0xABCDEF + rows])[0])
+    w_host = w.download()
+    field = rng.integers(0, 256, size=(2, n, 32), dtype=np.uint8)
+    field[:, :, 31] &= 0x3F
+    signed = rng.integers(-(1 << 62), 1 << 62, size=n)
+    signed[: n // 2] >>= 50  # the usual short values beside long ones
+    signed[0] = -(1 << 63)
+    counts = rng.integers(0, 1 << 32, size=n, dtype=np.uint32)
+    cols = [be.upload(field[0], KIND_FR), be.upload(field[1], KIND_FR_MONT), be.upload(signed, KIND_I64), be.upload(counts, KIND_U32)]
+    host = np.stack([field[0], field[1], ora.fr_from_i64(signed), ora.fr_from_i64(counts.astype(np.int64))])
+    host[:, rows:] = 0
+    rotations = (0, 1, n - 1)[:points]
+    want = ora.eval_rotations(host, w_host, rotations)
+    for _ in range(2):  # the second call finds the columns' counters as the first left them
+        assert np.array_equal(be.eval_batch(cols, rows, log2n, w, rotations), want)
+    assert np.array_equal(be.eval_batch(cols * 17, rows, log2n, w, rotations), np.tile(want, (1, 17, 1)))
