@@ -255,6 +255,21 @@ typedef struct gzk_scan_job
     gzk_buf* out;
 } gzk_scan_job;
 int gzk_running_sums_batch(gzk_ctx* ctx, const gzk_scan_job* jobs, size_t job_count);
+/* The same with integer keys for the lookups and route edges whose index[i].x is set (index NULL: for none): their
+ * inverses are fetched from the inverted table as in gzk_logup_accumulator_indexed (table = job.c0, whose queries,
+ * job.c1, and selectors, c3 and c4, are not read) and gzk_route_edge_accumulator_indexed (table = index.table, x the
+ * row that an edge's query is; job.c0 is not read), instead of one inversion per row. */
+typedef struct gzk_scan_index
+{
+    const gzk_buf* x;
+    const gzk_buf* y;
+    const gzk_buf* table;
+    const gzk_buf* table_y;
+    int64_t x_min;
+    size_t band;
+    size_t table_size;
+} gzk_scan_index;
+int gzk_running_sums_batch_indexed(gzk_ctx* ctx, const gzk_scan_job* jobs, const gzk_scan_index* index, size_t job_count);
 
 /* ---- a8: segmented prefix states over the dst-sorted edge list ------------------------
  * out[0] = v[0]; out[i] = q_new[i] ? v[i] : out[i-1] + v[i].  q_new must hold only

@@ -101,17 +101,16 @@ namespace gzk
 
         // inv_out[t] = 1/(table[t] + beta) in Montgomery form, t < count: the per-CTA batch inversion of the
         // main pass on its own (each CTA inverts the product of its 512 denominators).
-        __global__ void __launch_bounds__(kThreads) shifted_inverse_kernel(ScanArgs a, Fr* inv_out)
+        __device__ __forceinline__ void shifted_inverse_body(const ScanArgs& a, const ColRef& table, uint64_t count, uint32_t block, Fr* inv_out, BatchInvertShared<kThreads>& sh)
         {
-            __shared__ BatchInvertShared<kThreads> sh;
-            const uint64_t base = static_cast<uint64_t>(blockIdx.x) * kChunk + static_cast<uint64_t>(threadIdx.x) * kElems;
+            const uint64_t base = static_cast<uint64_t>(block) * kChunk + static_cast<uint64_t>(threadIdx.x) * kElems;
             Fr d[kElems], pre[kElems];
             Fr mine = Fr::one();
 #pragma unroll
             for (int j = 0; j < kElems; ++j)
             {
                 const uint64_t e = base + j;
-                d[j] = e < a.count ? add(col_load_stored(a.c0, e), beta_for(a, a.c0)) : Fr::one();
+                d[j] = e < count ? add(col_load_stored(table, e), beta_for(a, table)) : Fr::one();
                 pre[j] = mine;
                 mine = mul(mine, d[j]);
             }
@@ -124,8 +123,13 @@ namespace gzk
                 const uint64_t e = base + j;
                 const Fr inverse = mul(rest, pre[j]);
                 if (j > 0) rest = mul(rest, d[j]);
-                if (e < a.count) store_fr(inv_out + e, fix_scale(inverse, -deficit(a.c0)));
+                if (e < count) store_fr(inv_out + e, fix_scale(inverse, -deficit(table)));
             }
+        }
+        __global__ void __launch_bounds__(kThreads) shifted_inverse_kernel(ScanArgs a, Fr* inv_out)
+        {
+            __shared__ BatchInvertShared<kThreads> sh;
+            shifted_inverse_body(a, a.c0, a.count, blockIdx.x, inv_out, sh);
         }
 
         // LogUp rows with only one side switched on by its 0/1 selector (almost all of them: the table
@@ -553,8 +557,8 @@ namespace gzk
 
         // Fix-up that derives the offset of its chunk from the raw CTA aggregates itself (every
         // CTA re-adds at most a few thousand 32-byte values from L2), which saves the separate
-        // single-CTA scan of the aggregates when there are few of them.  A CTA covers kThreads
-        // consecutive outputs, all inside one chunk of the main pass.
+        // single-CTA scan of the aggregates when there are few of them.  A CTA covers one chunk of the main
+        // pass, kElems outputs per thread (a quarter of a chunk re-added the same aggregates four times as often).
         struct FixupShared
         {
             Fr warp_slots[kWarps];
@@ -566,9 +570,8 @@ namespace gzk
         {
             Fr* warp_slots = sh.warp_slots;
             int& last_start = sh.last_start;
-            const uint64_t first = static_cast<uint64_t>(block) * kThreads;
-            const uint64_t idx = first + threadIdx.x;
-            const uint32_t chunk = static_cast<uint32_t>(first / kChunk);
+            const uint64_t first = static_cast<uint64_t>(block) * kChunk;
+            const uint32_t chunk = block;
             if (OP == kSegmented)
             {
                 if (chunk == 0) return;
@@ -584,15 +587,20 @@ namespace gzk
                 Fr part = Fr::zero();
                 for (uint32_t i = from + threadIdx.x; i < chunk; i += kThreads) part = add(part, load_fr(a.agg_value + i));
                 const Fr offset = cta_sum(part, warp_slots);
-                if (idx < a.n && static_cast<uint32_t>(idx - static_cast<uint64_t>(chunk) * kChunk) < a.agg_first[chunk])
-                    store_fr(a.out + idx, add(load_fr_plain(a.out + idx), offset));
+                const uint32_t restart = a.agg_first[chunk];
+#pragma unroll
+                for (uint32_t j = 0; j < kElems; ++j)
+                {
+                    const uint32_t at = j * kThreads + threadIdx.x;
+                    if (first + at < a.n && at < restart) store_fr(a.out + first + at, add(load_fr_plain(a.out + first + at), offset));
+                }
                 return;
             }
             // out[idx] for 1 <= idx <= count belongs to chunk (idx - 1) / kChunk: the CTA's first output sits
-            // one chunk lower when the CTA starts on a chunk boundary
-            const bool needs_total = first + kThreads > a.count + 1 || block == 0;
+            // one chunk lower
+            const bool needs_total = first + kChunk > a.count + 1 || block == 0;
             Fr before = Fr::zero(), rest = Fr::zero();
-            const uint32_t limit = needs_total ? ctas : chunk;
+            const uint32_t limit = needs_total ? ctas : (chunk < ctas ? chunk : ctas);
             for (uint32_t i = threadIdx.x; i < limit; i += kThreads)
             {
                 const Fr v = load_fr(a.agg_value + i);
@@ -605,25 +613,30 @@ namespace gzk
             Fr total = offset;
             if (needs_total) total = add(offset, cta_sum(rest, warp_slots));
             if (block == 0 && threadIdx.x == 0) store_fr(a.total, total);
-            if (idx >= a.n) return;
-            if (idx == 0)
+#pragma unroll
+            for (uint32_t j = 0; j < kElems; ++j)
             {
-                store_fr(a.out, Fr::zero());
-            }
-            else if (idx <= a.count)
-            {
-                if (idx - 1 >= static_cast<uint64_t>(chunk) * kChunk)
+                const uint64_t idx = first + j * kThreads + threadIdx.x;
+                if (idx >= a.n) return;
+                if (idx == 0)
                 {
-                    if (chunk != 0) store_fr(a.out + idx, add(load_fr_plain(a.out + idx), offset));
+                    store_fr(a.out, Fr::zero());
                 }
-                else if (chunk >= 2)
+                else if (idx <= a.count)
                 {
-                    store_fr(a.out + idx, add(load_fr_plain(a.out + idx), sub(offset, load_fr(a.agg_value + (chunk - 1)))));
+                    if (idx - 1 >= first)
+                    {
+                        if (chunk != 0) store_fr(a.out + idx, add(load_fr_plain(a.out + idx), offset));
+                    }
+                    else if (chunk >= 2)
+                    {
+                        store_fr(a.out + idx, add(load_fr_plain(a.out + idx), sub(offset, load_fr(a.agg_value + (chunk - 1)))));
+                    }
                 }
-            }
-            else
-            {
-                store_fr(a.out + idx, total);
+                else
+                {
+                    store_fr(a.out + idx, total);
+                }
             }
         }
 
@@ -647,12 +660,25 @@ namespace gzk
             int op;
             uint32_t main_begin, main_ctas;    // CTAs of the main pass: [main_begin, main_begin + main_ctas)
             uint32_t fix_begin, fix_ctas;      // CTAs of the fix-up pass
+            uint32_t inv_begin, inv_ctas;      // CTAs of the table inversion (indexed jobs; the table is args.c3)
         };
         struct BatchTable
         {
             BatchJob jobs[kMaxBatchJobs];
             uint32_t count;
         };
+
+        // The inverted tables of the indexed jobs of a batch, side by side
+        __global__ void __launch_bounds__(kThreads) scan_batch_inverse_kernel(const BatchTable* table)
+        {
+            __shared__ BatchInvertShared<kThreads> sh;
+            uint32_t j = 0;
+            while (j + 1 < table->count && blockIdx.x >= table->jobs[j + 1].inv_begin) ++j;
+            const BatchJob& job = table->jobs[j];
+            const uint32_t block = blockIdx.x - job.inv_begin;
+            if (block >= job.inv_ctas) return;
+            shifted_inverse_body(job.args, job.args.c3, job.args.table_size, block, const_cast<Fr*>(job.args.inv_table), sh);
+        }
 
         __global__ void __launch_bounds__(kThreads) scan_batch_main_kernel(const BatchTable* table)
         {
@@ -668,6 +694,8 @@ namespace gzk
             case kRouteNode: scan_main_body<kRouteNode, true>(job.args, block, sh); break;
             case kRouteEdge: scan_main_body<kRouteEdge, true>(job.args, block, sh); break;
             case kProduct: scan_main_body<kProduct, true>(job.args, block, sh); break;
+            case kLogupIndexed: scan_main_body<kLogupIndexed, false>(job.args, block, sh); break;
+            case kRouteEdgeIndexed: scan_main_body<kRouteEdgeIndexed, false>(job.args, block, sh); break;
             default: scan_main_body<kSegmented, true>(job.args, block, sh); break;
             }
         }
@@ -685,7 +713,9 @@ namespace gzk
             case kLogup: scan_fixup_fused_body<kLogup>(job.args, job.main_ctas, block, sh); break;
             case kRouteNode: scan_fixup_fused_body<kRouteNode>(job.args, job.main_ctas, block, sh); break;
             case kRouteEdge: scan_fixup_fused_body<kRouteEdge>(job.args, job.main_ctas, block, sh); break;
-            case kProduct: scan_fixup_fused_body<kProduct>(job.args, job.main_ctas, block, sh); break;
+            case kProduct:
+            case kLogupIndexed:
+            case kRouteEdgeIndexed: scan_fixup_fused_body<kProduct>(job.args, job.main_ctas, block, sh); break;
             default: scan_fixup_fused_body<kSegmented>(job.args, job.main_ctas, block, sh); break;
             }
         }
@@ -736,7 +766,7 @@ namespace gzk
                 {
                     LaunchScope scope(ctx, "scan_fixup");
                     const uint64_t outputs = args.n > 0 ? args.n : 1;
-                    scan_fixup_fused_kernel<OP><<<static_cast<unsigned>((outputs + kThreads - 1) / kThreads), kThreads, 0, ctx->stream>>>(args, ctas);
+                    scan_fixup_fused_kernel<OP><<<static_cast<unsigned>((outputs + kChunk - 1) / kChunk), kThreads, 0, ctx->stream>>>(args, ctas);
                 }
             }
             else
@@ -788,6 +818,29 @@ namespace gzk
 
 using namespace gzk;
 
+static bool integer_keys(const gzk_buf* b, size_t count) { return b != nullptr && (b->kind == GZK_KIND_I64 || b->kind == GZK_KIND_U32) && b->count >= count; }
+
+// The arguments of an indexed lookup: keys, multiplicities and the shape of the table (job.c0, left in args->c3).
+static int index_logup(gzk_ctx* ctx, const gzk_scan_job& job, const gzk_scan_index& index, size_t active_count, ScanArgs* args)
+{
+    const bool has_y = index.y != nullptr;
+    const size_t table_size = index.table_size, band = index.band;
+    if (band == 0 || band > 64 || table_size == 0 || table_size % band != 0 || table_size > job.domain_size || has_y != (index.table_y != nullptr) || (!has_y && band != 1))
+        return fail(ctx, GZK_E_INVALID, "logup (indexed): the table must hold a whole number of bands and fit the column");
+    if (!col_ok(job.c0, table_size) || job.c2 == nullptr || job.c2->kind != GZK_KIND_U32 || job.c2->count < table_size || !integer_keys(index.x, active_count) ||
+        (has_y && (!integer_keys(index.y, active_count) || index.table_y->kind != GZK_KIND_I64 || index.table_y->count < table_size)))
+        return fail(ctx, GZK_E_INVALID, "lookup accumulator input size mismatch");
+    args->c0 = ref(index.x);
+    args->c1 = has_y ? ref(index.y) : ref(index.x);
+    args->c2 = ref(job.c2);
+    args->c3 = ref(job.c0);
+    args->table_y = has_y ? static_cast<const long long*>(index.table_y->dptr) : nullptr;
+    args->table_size = table_size;
+    args->x_min = static_cast<long long>(index.x_min);
+    args->band = static_cast<uint32_t>(band);
+    return GZK_OK;
+}
+
 extern "C"
 {
     int gzk_logup_accumulator_indexed(gzk_ctx* ctx, const gzk_buf* table, const gzk_buf* multiplicity, const gzk_buf* x, const gzk_buf* y,
@@ -798,40 +851,40 @@ extern "C"
         if (beta == nullptr || !out_ok(out, n)) return fail(ctx, GZK_E_INVALID, "logup: output must be a Montgomery buffer of n elements");
         if (n > 0 && active_count > n - 1) active_count = n - 1;  // lookup.cpp:117
         if (n == 0) return GZK_OK;
-        const bool has_y = y != nullptr;
-        auto keys_ok = [&](const gzk_buf* b) { return b != nullptr && (b->kind == GZK_KIND_I64 || b->kind == GZK_KIND_U32) && b->count >= active_count; };
-        if (band == 0 || band > 64 || table_size == 0 || table_size % band != 0 || table_size > n || has_y != (table_y != nullptr) || (!has_y && band != 1))
-            return fail(ctx, GZK_E_INVALID, "logup (indexed): the table must hold a whole number of bands and fit the column");
-        if (!col_ok(table, table_size) || multiplicity == nullptr || multiplicity->kind != GZK_KIND_U32 || multiplicity->count < table_size || !keys_ok(x) ||
-            (has_y && (!keys_ok(y) || table_y->kind != GZK_KIND_I64 || table_y->count < table_size)))
-            return fail(ctx, GZK_E_INVALID, "lookup accumulator input size mismatch");
         GZK_CUDA_TRY(ctx, cudaSetDevice(ctx->device));
         ScanArgs args{};
-        int rc = load_scalar(ctx, beta, &args.beta, &args.beta_canon);
+        gzk_scan_job job{};
+        job.c0 = table;
+        job.c2 = multiplicity;
+        job.domain_size = n;
+        gzk_scan_index index{};
+        index.x = x;
+        index.y = y;
+        index.table_y = table_y;
+        index.x_min = x_min;
+        index.band = band;
+        index.table_size = table_size;
+        int rc = index_logup(ctx, job, index, active_count, &args);
+        if (rc != GZK_OK) return rc;
+        rc = load_scalar(ctx, beta, &args.beta, &args.beta_canon);
         if (rc != GZK_OK) return rc;
         void* scratch = nullptr;
         if ((rc = ensure_scratch(ctx, 1, table_size * sizeof(Fr), &scratch)) != GZK_OK) return rc;
         // pass 0: the inverses of the shifted table
-        args.c0 = ref(table);
-        args.count = table_size;
-        args.status = ctx->d_status;
+        ScanArgs inverses = args;
+        inverses.c0 = args.c3;
+        inverses.count = table_size;
+        inverses.status = ctx->d_status;
         if ((rc = begin_call(ctx)) != GZK_OK) return rc;
         {
             LaunchScope scope(ctx, "logup_table_inverses");
-            shifted_inverse_kernel<<<static_cast<unsigned>((table_size + kChunk - 1) / kChunk), kThreads, 0, ctx->stream>>>(args, static_cast<Fr*>(scratch));
+            shifted_inverse_kernel<<<static_cast<unsigned>((table_size + kChunk - 1) / kChunk), kThreads, 0, ctx->stream>>>(inverses, static_cast<Fr*>(scratch));
         }
         GZK_CUDA_TRY(ctx, cudaGetLastError());
-        args.c0 = ref(x);
-        args.c1 = has_y ? ref(y) : ref(x);
-        args.c2 = ref(multiplicity);
         args.count = active_count;
         args.n = n;
         args.out = static_cast<Fr*>(out->dptr);
         args.inv_table = static_cast<const Fr*>(scratch);
-        args.table_y = has_y ? static_cast<const long long*>(table_y->dptr) : nullptr;
-        args.table_size = table_size;
-        args.x_min = static_cast<long long>(x_min);
-        args.band = static_cast<uint32_t>(band);
         return run_scan<kLogupIndexed>(ctx, args, false, nullptr, true);
     }
 
@@ -956,6 +1009,11 @@ extern "C"
 
     int gzk_running_sums_batch(gzk_ctx* ctx, const gzk_scan_job* jobs, size_t job_count)
     {
+        return gzk_running_sums_batch_indexed(ctx, jobs, nullptr, job_count);
+    }
+
+    int gzk_running_sums_batch_indexed(gzk_ctx* ctx, const gzk_scan_job* jobs, const gzk_scan_index* index, size_t job_count)
+    {
         if (ctx == nullptr) return GZK_E_INVALID;
         if (job_count == 0) return GZK_OK;
         if (jobs == nullptr) return fail(ctx, GZK_E_INVALID, "running_sums_batch: null job list");
@@ -970,9 +1028,9 @@ extern "C"
             size_t scratch_frs = 0, scratch_u32 = 0;
             struct Layout
             {
-                size_t fr_at, u32_at;
+                size_t fr_at, u32_at, inverse_at;
             } layout[kMaxBatchJobs];
-            uint32_t main_total = 0, fix_total = 0;
+            uint32_t main_total = 0, fix_total = 0, inv_total = 0;
             while (done < job_count && table.count < kMaxBatchJobs)
             {
                 const gzk_scan_job& j = jobs[done];
@@ -988,10 +1046,17 @@ extern "C"
                     ++done;
                     continue;
                 }
+                const gzk_scan_index* x = index != nullptr && index[done].x != nullptr ? index + done : nullptr;
+                if (x != nullptr && j.op != GZK_SCAN_LOGUP && j.op != GZK_SCAN_ROUTE_EDGE) return fail(ctx, GZK_E_INVALID, "running_sums_batch: only lookups and route edges take keys");
                 switch (j.op)
                 {
                 case GZK_SCAN_LOGUP:
                     if (count > n - 1) count = n - 1;
+                    if (x != nullptr)
+                    {
+                        if (j.beta == nullptr || (rc = index_logup(ctx, j, *x, count, &a)) != GZK_OK) return j.beta == nullptr ? fail(ctx, GZK_E_INVALID, "lookup accumulator input size mismatch") : rc;
+                        break;
+                    }
                     if (j.beta == nullptr || !col_ok(j.c0, count) || !col_ok(j.c1, count) || !col_ok(j.c2, count) || !col_ok(j.c3, count) || !col_ok(j.c4, count))
                         return fail(ctx, GZK_E_INVALID, "lookup accumulator input size mismatch");
                     a.c0 = ref(j.c0);
@@ -1008,6 +1073,15 @@ extern "C"
                     break;
                 case GZK_SCAN_ROUTE_EDGE:
                     if (count >= n) return fail(ctx, GZK_E_INVALID, "route accumulator needs valid_length < domain_size");
+                    if (x != nullptr)
+                    {
+                        if (j.beta == nullptr || x->table_size == 0 || !col_ok(x->table, x->table_size) || !integer_keys(x->x, count))
+                            return fail(ctx, GZK_E_INVALID, "route accumulator input size mismatch");
+                        a.c0 = ref(x->x);
+                        a.c3 = ref(x->table);
+                        a.table_size = x->table_size;
+                        break;
+                    }
                     if (j.beta == nullptr || !col_ok(j.c0, count)) return fail(ctx, GZK_E_INVALID, "route edge accumulator input size mismatch");
                     a.c0 = ref(j.c0);
                     break;
@@ -1035,14 +1109,19 @@ extern "C"
                 if (ctas > 2048) return fail(ctx, GZK_E_INVALID, "running_sums_batch: at most 2^20 rows per job; use the single-column entry point for longer columns");
                 b.op = j.op == GZK_SCAN_LOGUP ? kLogup : j.op == GZK_SCAN_ROUTE_NODE ? kRouteNode : j.op == GZK_SCAN_ROUTE_EDGE ? kRouteEdge
                        : j.op == GZK_SCAN_ZKMAP ? kProduct : kSegmented;
+                if (x != nullptr) b.op = j.op == GZK_SCAN_LOGUP ? kLogupIndexed : kRouteEdgeIndexed;
+                b.inv_begin = inv_total;
+                b.inv_ctas = x != nullptr ? static_cast<uint32_t>((a.table_size + kChunk - 1) / kChunk) : 0u;
+                inv_total += b.inv_ctas;
                 b.main_begin = main_total;
                 b.main_ctas = static_cast<uint32_t>(ctas);
                 b.fix_begin = fix_total;
-                b.fix_ctas = static_cast<uint32_t>((n + kThreads - 1) / kThreads);
+                b.fix_ctas = static_cast<uint32_t>((n + kChunk - 1) / kChunk);
                 main_total += b.main_ctas;
                 fix_total += b.fix_ctas;
-                layout[table.count] = {scratch_frs, scratch_u32};
+                layout[table.count] = {scratch_frs, scratch_u32, scratch_frs + ctas + 1};
                 scratch_frs += ctas + 1;       // aggregates + total
+                if (x != nullptr) scratch_frs += a.table_size;
                 scratch_u32 += 2 * ctas;       // flags + first-restart marks
                 ++table.count;
                 ++done;
@@ -1060,11 +1139,18 @@ extern "C"
                 a.cta_products = nullptr;  // every CTA inverts its own product
                 a.agg_value = fr_base + layout[t].fr_at;
                 a.total = a.agg_value + ctas;
+                if (table.jobs[t].inv_ctas != 0) a.inv_table = fr_base + layout[t].inverse_at;
                 a.agg_flag = u32_base + layout[t].u32_at;
                 a.agg_first = a.agg_flag + ctas;
             }
             // the table travels from pageable memory of this call: the copy is staged before the call returns
             GZK_CUDA_TRY(ctx, cudaMemcpyAsync(scratch, &table, sizeof(BatchTable), cudaMemcpyHostToDevice, ctx->stream));
+            if (inv_total != 0)
+            {
+                LaunchScope scope(ctx, "scan_batch_inverse");
+                scan_batch_inverse_kernel<<<inv_total, kThreads, 0, ctx->stream>>>(static_cast<const BatchTable*>(scratch));
+            }
+            GZK_CUDA_TRY(ctx, cudaGetLastError());
             {
                 LaunchScope scope(ctx, "scan_batch_main");
                 scan_batch_main_kernel<<<main_total, kThreads, 0, ctx->stream>>>(static_cast<const BatchTable*>(scratch));

@@ -93,6 +93,7 @@ namespace gatzk_flow
         ColP key_x, key_y, table_y;
         std::int64_t x_min = 0;
         std::size_t band = 0, table_size = 0;
+        bool gathered = false;  // every query is the table row its key points at
     };
 
     // The compute backend: every call is one data-parallel leaf of the hot path.
@@ -650,7 +651,7 @@ namespace gatzk_flow
             ColP table, query, node_acc, edge_acc;  // the routed total is node_acc[node_count]
         };
         Route build_route(const std::vector<ColP>& node_cols, const std::vector<ColP>& edge_cols, const Fe& eta, const ColP& multiplicity,
-                          const Fe& beta);
+                          const Fe& beta, bool gathered);
         struct HeadWitness
         {
             ColP h_prime, h_agg_pre, h_agg;                       // I64 matrices node_count x width
@@ -1287,13 +1288,15 @@ namespace gatzk_flow
         job.x_min = x_min;
         job.band = band;
         job.table_size = table_size;
+        job.gathered = true;
         return out;
     }
 
     // route packs + build_route_trace (trace.cpp:1776-1794): table = sum_j eta^j node_cols[j],
-    // query = sum_j eta^j edge_cols[j]
+    // query = sum_j eta^j edge_cols[j].  `gathered`: the edge columns are the node columns at the edges' endpoints (the
+    // source route packs (id, E_src) for the nodes and (src, H*) for the edges, as the reference does)
     inline ProverFlow::Route ProverFlow::build_route(const std::vector<ColP>& node_cols, const std::vector<ColP>& edge_cols, const Fe& eta,
-                                                     const ColP& multiplicity, const Fe& beta)
+                                                     const ColP& multiplicity, const Fe& beta, bool gathered)
     {
         const Domain& n = dom_.at("N");
         const auto eta_powers = powers_host(eta, node_cols.size());
@@ -1313,6 +1316,7 @@ namespace gatzk_flow
             job.key_x = edge_cols.front();
             job.table_y = out.table;
             job.table_size = n_nodes_;
+            job.gathered = gathered;
         }
         return out;
     }
@@ -1543,7 +1547,7 @@ namespace gatzk_flow
         const ColP psq = be_.alloc(kFrMont, es_);
         queue_scan(ScanJob::kGroupPrefix, w_psq, q_new_, nullptr, nullptr, nullptr, es_, es_, Fe{}, psq);
         // the source route packs ids + eta * value with powers(eta, 2) = {1, eta} (trace.cpp:2737-2772)
-        const Route src_route = build_route({ids_i64_, w.e_src}, {src_i64_, h_star_edge}, eta_src, src_multiplicity_, beta_src);
+        const Route src_route = build_route({ids_i64_, w.e_src}, {src_i64_, h_star_edge}, eta_src, src_multiplicity_, beta_src, false);
 
         const std::size_t dd = dom_.at("d").size, di = dom_.at("in").size;
         commit_batch({column_item(prefix + "a_proj", proj.a, "in", di), column_item(prefix + "b_proj", proj.b, "in", di),
@@ -1574,7 +1578,7 @@ namespace gatzk_flow
         absorb_dyn(t, prefix + "T_psq_edge");
         const Fe eta_t = challenge(t, "eta_t_h" + h);
         const Fe beta_t = challenge(t, "beta_t_h" + h);
-        const Route t_route = build_route({ids_i64_, t_psq}, {dst_i64_, t_psq_edge}, eta_t, dst_multiplicity_, beta_t);
+        const Route t_route = build_route({ids_i64_, t_psq}, {dst_i64_, t_psq_edge}, eta_t, dst_multiplicity_, beta_t, true);
         absorb_dyn(t, prefix + "H_agg_pre");
         absorb_dyn(t, prefix + "H_agg_pre_star");
         const Fe y_agg_pre = challenge(t, "y_agg_pre_h" + h);
@@ -1601,7 +1605,7 @@ namespace gatzk_flow
                                              eta_elu, beta_elu, q_tbl_elu_, q_qry_elu_);
         const Route dst_route = build_route({ids_i64_, w.e_dst, w.m, w.sum, w.inv, h_agg_star},
                                             {dst_i64_, w.e_dst_edge, w.m_edge, w.sum_edge, w.inv_edge, h_agg_star_edge}, eta_dst, dst_multiplicity_,
-                                            beta_dst);
+                                            beta_dst, true);
 
         commit_batch({column_item(prefix + "a_agg_pre", agg_pre_b.a, "d", dd), column_item(prefix + "b_agg_pre", agg_pre_b.b, "d", dd),
                       column_item(prefix + "Acc_agg_pre", agg_pre_b.acc, "d", dd), column_item(prefix + "a_agg", agg_b.a, "d", dd),

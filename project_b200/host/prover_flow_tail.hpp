@@ -125,7 +125,7 @@ namespace gatzk_flow
         const ColP y_prime_star_edge = to_edges(y_prime_star, src_u32_), y_star_edge = to_edges(y_star, dst_u32_);
         const Fe eta_src = challenge(t, cname("eta_src_out"));
         const Fe beta_src = challenge(t, cname("beta_src_out"));
-        const Route src_route = build_route({ids_i64_, w.e_src}, {src_i64_, y_prime_star_edge}, eta_src, src_multiplicity_, beta_src);
+        const Route src_route = build_route({ids_i64_, w.e_src}, {src_i64_, y_prime_star_edge}, eta_src, src_multiplicity_, beta_src, false);
 
         const std::size_t lrelu_size = lrelu_bound_ * 2 + 1;
         const Lookup lrelu = build_pair_lookup(t_l_x_, t_l_y_, lrelu_size, -static_cast<std::int64_t>(lrelu_bound_), 1, w.s, w.z, n_edges_, eta_l,
@@ -169,7 +169,7 @@ namespace gatzk_flow
         absorb_dyn(t, prefix + "T_edge");
         const Fe eta_t = challenge(t, cname("eta_t_out"));
         const Fe beta_t = challenge(t, cname("beta_t_out"));
-        const Route t_route = build_route({ids_i64_, t_out}, {dst_i64_, t_out_edge}, eta_t, dst_multiplicity_, beta_t);
+        const Route t_route = build_route({ids_i64_, t_out}, {dst_i64_, t_out_edge}, eta_t, dst_multiplicity_, beta_t, true);
         absorb_dyn(t, y_label);
         absorb_dyn(t, prefix + "Y_star");
         const Fe y_out_star = challenge(t, cname("y_out_star"));
@@ -190,7 +190,7 @@ namespace gatzk_flow
         const Fe eta_dst = challenge(t, cname("eta_dst_out"));
         const Fe beta_dst = challenge(t, cname("beta_dst_out"));
         const Route dst_route = build_route({ids_i64_, w.e_dst, w.m, w.sum, w.inv, y_star},
-                                            {dst_i64_, w.e_dst_edge, w.m_edge, w.sum_edge, w.inv_edge, y_star_edge}, eta_dst, dst_multiplicity_, beta_dst);
+                                            {dst_i64_, w.e_dst_edge, w.m_edge, w.sum_edge, w.inv_edge, y_star_edge}, eta_dst, dst_multiplicity_, beta_dst, true);
         const std::size_t dc = cd.size, dcat = dom_.at("cat").size;
         commit_batch({column_item(prefix + "Table_t", t_route.table, "N", n.size), column_item(prefix + "Query_t", t_route.query, "edge", es_),
                       column_item(prefix + "m_t", dst_multiplicity_, "N", n.size), column_item(prefix + "R_t_node", t_route.node_acc, "N", n.size),

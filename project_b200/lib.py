@@ -67,6 +67,11 @@ class _ScanJob(ctypes.Structure):
                 ("c4", ctypes.c_void_p), ("count", ctypes.c_size_t), ("domain_size", ctypes.c_size_t), ("beta", ctypes.c_void_p), ("out", ctypes.c_void_p)]
 
 
+class _ScanIndex(ctypes.Structure):
+    _fields_ = [("x", ctypes.c_void_p), ("y", ctypes.c_void_p), ("table", ctypes.c_void_p), ("table_y", ctypes.c_void_p), ("x_min", ctypes.c_int64),
+                ("band", ctypes.c_size_t), ("table_size", ctypes.c_size_t)]
+
+
 SCAN_LOGUP, SCAN_ROUTE_NODE, SCAN_ROUTE_EDGE, SCAN_ZKMAP, SCAN_GROUP_PREFIX = 0, 1, 2, 3, 4
 
 
@@ -281,13 +286,14 @@ class Backend:
                                                                 _sz(domain_size), _ptr(_fr(beta)), out.handle))
         return out
 
-    def running_sums_batch(self, jobs):
-        """jobs: list of (op, [input Buffers], count, domain_size, beta or None, out Buffer): gzk_running_sums_batch."""
+    def running_sums_batch(self, jobs, keys=None):
+        """jobs: list of (op, [input Buffers], count, domain_size, beta or None, out Buffer): gzk_running_sums_batch.
+        keys: for each job None or a dict of the fields of gzk_scan_index (gzk_running_sums_batch_indexed)."""
         raw = (_ScanJob * len(jobs))()
         keep = []
         for r, (op, cols, count, domain_size, beta, out) in zip(raw, jobs):
             r.op = op
-            handles = [c.handle for c in cols] + [None] * (5 - len(cols))
+            handles = [c.handle if c is not None else None for c in cols] + [None] * (5 - len(cols))
             r.c0, r.c1, r.c2, r.c3, r.c4 = handles
             r.count, r.domain_size = int(count), int(domain_size)
             if beta is not None:
@@ -295,7 +301,14 @@ class Backend:
                 keep.append(b)
                 r.beta = b.ctypes.data
             r.out = out.handle
-        self._check(self.lib.gzk_running_sums_batch(self.ctx, raw, _sz(len(jobs))))
+        if keys is None:
+            self._check(self.lib.gzk_running_sums_batch(self.ctx, raw, _sz(len(jobs))))
+            return
+        index = (_ScanIndex * len(jobs))()
+        for r, fields in zip(index, keys):
+            for name, value in (fields or {}).items():
+                setattr(r, name, getattr(value, "handle", value))
+        self._check(self.lib.gzk_running_sums_batch_indexed(self.ctx, raw, index, _sz(len(jobs))))
 
     def group_prefix_state(self, values, q_new, n, out=None):
         out = out or self.alloc(KIND_FR_MONT, n)
@@ -383,6 +396,20 @@ class Backend:
         out = self.alloc(KIND_U32, domain_size)
         self._check(self.lib.gzk_first_zero_marker(self.ctx, delta.handle, group_begin.handle, group_end.handle, _sz(groups), _sz(domain_size), out.handle))
         return out
+
+    def download_elements(self, bufs, indices):
+        """Element indices[i] of bufs[i] (field-element buffers), canonical: gzk_buf_download_elements."""
+        handles = (ctypes.c_void_p * len(bufs))(*[b.handle for b in bufs])
+        index = np.ascontiguousarray(indices, dtype=np.uint64)
+        out = np.zeros((len(bufs), 32), dtype=np.uint8)
+        self._check(self.lib.gzk_buf_download_elements(self.ctx, handles, _ptr(index), _sz(len(bufs)), _ptr(out)))
+        return out
+
+    def g1_fixed_base_mul_download(self, base, scalars, count):
+        """The scalars of a device buffer and the points they give, on the host: gzk_g1_fixed_base_mul_download."""
+        values, points = np.zeros((count, 32), dtype=np.uint8), np.zeros((count, 96), dtype=np.uint8)
+        self._check(self.lib.gzk_g1_fixed_base_mul_download(self.ctx, _ptr(np.ascontiguousarray(base)), scalars.handle, _sz(count), _ptr(values), _ptr(points)))
+        return values, points
 
     def g1_mul_same_base(self, base, scalars):
         base = np.ascontiguousarray(base, dtype=np.uint8).reshape(-1)

@@ -597,3 +597,41 @@ def test_matrix_horner_block_sums_on_the_tensor_path(be):
     x = fr_array([int(rng.integers(2, 1 << 62))])
     got = be.matrix_horner(be.upload(vals, KIND_I64), rows, cols, x)
     assert np.array_equal(got, ora.matrix_row_major_eval(ora.fr_from_i64(vals).reshape(rows, cols, 32), x))
+
+
+@pytest.mark.parametrize("valid,n,has_y", [(1500, 2048, True), (9000, 9001, False), (70000, 1 << 17, True), (513, 1024, False)])
+def test_running_sums_batch_with_keys(be, valid, n, has_y):
+    """Lookups and route edges with integer keys in a batch, beside jobs without: the columns of the single-column builders."""
+    from project_b200 import KIND_FR, KIND_FR_MONT, KIND_I64, KIND_U32, GzkError
+    from project_b200.lib import SCAN_LOGUP, SCAN_ROUTE_EDGE, SCAN_ZKMAP
+
+    rng = np.random.default_rng(valid)
+    band, xs, x_min = (3, 70, -35) if has_y else (1, 200, -100)
+    table_size = xs * band
+    table_x = np.repeat(np.arange(x_min, x_min + xs, dtype=np.int64), band)
+    table_y = table_x * 7 + np.tile(np.arange(band, dtype=np.int64), xs) - 1
+    pick = rng.integers(0, table_size, size=valid)
+    beta = fr_array([int(rng.integers(1, 1 << 62))])
+    pad = lambda v: np.concatenate([v, np.zeros(n - v.size, dtype=np.int64)])
+    bx, by = be.upload(pad(table_x[pick]), KIND_I64), be.upload(pad(table_y[pick]), KIND_I64) if has_y else None
+    btx, bty = be.upload(pad(table_x), KIND_I64), be.upload(pad(table_y), KIND_I64) if has_y else None
+    mult = be.banded_lookup_multiplicity(bx, by, valid, x_min, band, bty, table_size, n)
+    table = be.linear_combination([btx, bty], np.concatenate([fr_array([1]), fr_array([99])]), table_size, n) if has_y else btx
+    nodes = max(2, valid // 5)
+    node_table = rand_fr(rng, nodes)
+    ends = np.concatenate([rng.integers(0, nodes, size=valid, dtype=np.uint32), np.zeros(n - valid, dtype=np.uint32)])
+    b_nodes, b_ends = be.upload(node_table, KIND_FR), be.upload(ends, KIND_U32)
+    a, b = be.upload(rand_fr(rng, n), KIND_FR), be.upload(rand_fr(rng, n), KIND_FR)
+    outs = [be.alloc(KIND_FR_MONT, n) for _ in range(4)]
+    lookup = {"x": bx, "y": by, "table_y": bty, "x_min": x_min, "band": band, "table_size": table_size}
+    jobs = [(SCAN_ZKMAP, [a, b], valid, n, None, outs[0]), (SCAN_LOGUP, [table, None, mult], valid, n, beta, outs[1]),
+            (SCAN_ROUTE_EDGE, [None], valid, n, beta, outs[2]), (SCAN_ZKMAP, [b, a], valid - 1, n, None, outs[3])]
+    be.running_sums_batch(jobs, [None, lookup, {"x": b_ends, "table": b_nodes, "table_size": nodes}, None])
+    assert np.array_equal(outs[1].download(), be.logup_accumulator_indexed(table, mult, bx, by, valid, x_min, band, bty, table_size, n, beta).download())
+    query = np.zeros((n, 32), dtype=np.uint8)
+    query[:valid] = node_table[ends[:valid]]
+    assert np.array_equal(outs[2].download(), ora.route_edge_accumulator(query, valid, beta))
+    for out, (l, r, count) in ((outs[0], (a, b, valid)), (outs[3], (b, a, valid - 1))):
+        assert np.array_equal(out.download(), be.zkmap_accumulator(l, r, count, n)[0].download())
+    with pytest.raises(GzkError):
+        be.running_sums_batch([(SCAN_ROUTE_EDGE, [None], valid, n, beta, outs[2])], [{"x": b_ends, "table": b_nodes, "table_size": nodes - 1 if ends[:valid].max() == nodes - 1 else int(ends[:valid].max())}])

@@ -209,3 +209,20 @@ def test_msm_plans(be, n, kind):
             table, used = be.msm_precompute(pts, n, bits)
             assert bytes(be.msm_precomputed(s, table, n, used)) == want
             table.free()
+
+
+@pytest.mark.parametrize("count", [1, 128, 129, 300])  # one launch of the gather, full, and several
+def test_read_back_of_single_elements_and_barrier_points(be, count):
+    from project_b200 import KIND_FR, KIND_FR_MONT, GzkError
+
+    rng = random.Random(count)
+    values = fr_array(pyref.rand_fr(rng, 400))
+    bufs = [be.upload(values, KIND_FR), be.upload(values, KIND_FR_MONT)]
+    picks = [rng.randrange(400) for _ in range(count)]
+    assert np.array_equal(be.download_elements([bufs[i % 2] for i in range(count)], picks), values[picks])
+    with pytest.raises(GzkError):
+        be.download_elements([bufs[0]], [400])
+    for buf in bufs:
+        got, points = be.g1_fixed_base_mul_download(G, buf, count)
+        assert np.array_equal(got, values[:count])
+        assert np.array_equal(points, ora.g1_mul_same_base(G, values[:count]))
