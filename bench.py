@@ -375,15 +375,15 @@ def main():
         peak, peak_src = 6650.0, "fallback"
     from project_b200.lib import measure_mac_peak
 
-    eval_ms = sum(v[1] for k, v in report.items() if k.startswith("eval_partial"))
-    eval_launches = sum(v[0] for k, v in report.items() if k.startswith("eval_partial"))
+    eval_ms = sum(v[1] for k, v in report.items() if k.startswith(("eval_partial", "eval_short")))
+    eval_launches = sum(v[0] for k, v in report.items() if k.startswith(("eval_partial", "eval_short")))
     achieved = work[0] / (eval_ms * 1e-3) / 1e9 if eval_ms > 0 else 0.0
     mac_peak = measure_mac_peak(local_rank, 2, 20000)  # 8x8-limb products per second
     limb_rate = work[1] / (eval_ms * 1e-3) if eval_ms > 0 else 0.0
     field_terms = max(0, (work[1] - 8 * work[2]) // 56)  # terms of field-element columns (64 limb products each; 8 for the others)
     roofline = {
         "bound": "hbm",
-        "kernel": "eval_partial_kernel / eval_integers_kernel (packed evaluation: commit tau-evaluations, quotient and opening evaluations; "
+        "kernel": "eval_partial_kernel / eval_integers_kernel / eval_short_kernel (packed evaluation: commit tau-evaluations, quotient and opening evaluations; "
                   "all launches of one proof, each timed by itself)",
         "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak if peak else None,
         "traffic": (537.0e6 + 4.5e6) / 536.9e6 * work[0] / max(1, eval_launches),

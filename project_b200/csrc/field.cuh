@@ -729,8 +729,8 @@ namespace gzk
     // to the full-length a, b and to the cofactors u, v.  ceil((2*bits-1)/31) such rounds
     // reach a = 0, b = 1, v = 1/value.  The cofactor update divides by 2^31 modulo the
     // modulus each round, so no correction is left at the end except the Montgomery one.
-    // About four times shorter as a dependent chain than inv_binary(); every batch inversion
-    // of the library ends in exactly one such serial inversion.  a must be non-zero (0 maps to 0).
+    // About four times shorter as a dependent chain than inv_binary().  For the host and for threads that invert
+    // each for themselves; where a CTA waits for one inversion, inv_quad() is the shorter chain.  a must be non-zero (0 maps to 0).
     template <typename Cfg>
     GZK_HD Fe<Cfg> inv(const Fe<Cfg>& value)
     {
